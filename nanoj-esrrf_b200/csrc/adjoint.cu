@@ -856,6 +856,7 @@ esrrf_status esrrf_adjoint::forward(const float* frames, float fwhm, float sens,
         a.F = T;
         a.int_weighting = 1;
         a.cg_out = C;
+        a.edge = Q;  // free in a loss-only evaluation
         AK(fht_rgc_fused(geo, tables, a, stream), "RGC");
     }
     recon_kernel<<<(unsigned)((P + 255) / 256), 256, 0, stream>>>(I, C, T, P, sens, R);

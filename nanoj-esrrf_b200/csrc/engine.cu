@@ -411,9 +411,11 @@ esrrf_status esrrf_handle::process_chunk(const void* src, bool is_u16, int F_now
     a.int_weighting = p.int_weighting;
     a.st = st;
     a.prev_out = d_prev_out;
+    a.own = d_gx;   // the gradient planes: only the plain kernel and read-back fill them with gradients
+    a.edge = d_gy;
     if (use_fused && !any_drift) {
+        launches += fht_pair_pays(geo, tables, a) ? 2 : 1;  // the paired taps and their cumulants
         CK(fht_rgc_fused(geo, tables, a, stream));
-        launches += 1;
     } else if (use_fused && d_drift) {
         // frames with drift: per-frame tap tables and shifted intensities, then the fused kernel
         // (the kernel samples the shifted intensities from its own tiles: no intensity planes)

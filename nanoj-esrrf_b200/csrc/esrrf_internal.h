@@ -123,6 +123,10 @@ struct FhtRgcArgs {
                                 // into groups across CTAs (the last group's values land here and
                                 // are copied to st.prev after the launch, so no group overwrites a
                                 // value another group still reads); null: one group
+    // planes [F][H][W] that let a launch take the paired-tap kernel (rgc_pair.cuh): each strip's own
+    // columns (per-frame mode: cg_out itself) and its terms for the neighbouring strips' columns
+    float* own = nullptr;
+    float* edge = nullptr;
 };
 
 cudaError_t fht_robx(const float* interp, int W, int H, int F, float* gx, float* gy,
@@ -134,7 +138,18 @@ struct FhtFusedTables {
     float* wdtab = nullptr;    // device [S*S] weight / distance
     int* jrange = nullptr;     // device [2*S]
     float* wsum = nullptr;     // device [H*W] per-pixel weight sums
+    // paired-tap kernel: (w, w/d) per column distance i and row distance |j| (0 .. R + 1 each), per i
+    // the largest |j| <= R in the disc (-1: none) and whether row distance R + 1 is in it
+    float2* ptab = nullptr;
+    signed char pJ[18] = {};
+    unsigned char pfar[18] = {};
+    int taps = 0;              // taps of the disc
 };
+// The paired-tap part of the tables; fht_rgc_fused takes that kernel where fht_pair_pays says so.
+cudaError_t fht_pair_tables(const FhtGeometry& g, FhtFusedTables& t, cudaStream_t stream);
+bool fht_pair_pays(const FhtGeometry& g, const FhtFusedTables& t, const FhtRgcArgs& a);
+cudaError_t fht_rgc_pair(const FhtGeometry& g, const FhtFusedTables& t, const FhtRgcArgs& a,
+                         cudaStream_t stream);
 cudaError_t fht_fused_tables(const FhtGeometry& g, int W, int H, FhtFusedTables& t,
                              cudaStream_t stream);
 void fht_fused_tables_free(FhtFusedTables& t);

@@ -244,6 +244,7 @@ cudaError_t fht_fused_tables(const FhtGeometry& g, int W, int H, FhtFusedTables&
     wsum_kernel<<<(unsigned)((wh + 255) / 256), 256, 0, stream>>>(t.wtab, g.r0, S, W, H, t.wsum);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
+    if ((e = fht_pair_tables(g, t, stream)) != cudaSuccess) return e;
     return cudaStreamSynchronize(stream);  // host tables above are stack temporaries
 }
 
@@ -252,11 +253,13 @@ void fht_fused_tables_free(FhtFusedTables& t) {
     cudaFree(t.wdtab);
     cudaFree(t.jrange);
     cudaFree(t.wsum);
+    cudaFree(t.ptab);
     t = FhtFusedTables();
 }
 
 cudaError_t fht_rgc_fused(const FhtGeometry& g, const FhtFusedTables& t, const FhtRgcArgs& a,
                           cudaStream_t stream) {
+    if (fht_pair_pays(g, t, a)) return fht_rgc_pair(g, t, a, stream);
     const fused::FusedParams fp{g.r0, g.sensitivity, t.wtab, t.wdtab, t.jrange, t.wsum};
     return fused::launch_fused_in<false, 4, 32>(g.S, g.r0, g.sensitivity, fp, fused::DriftParams{}, a, stream);
 }

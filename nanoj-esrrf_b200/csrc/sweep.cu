@@ -176,6 +176,7 @@ struct Shard {
     InterpScratch scratch;
     float* d_interp = nullptr;  // [T][HM][WM] for the largest magnification
     float* d_cg = nullptr;
+    float* d_edge = nullptr;    // FHT sweep without drift: the paired-tap kernel's second plane [T][HM][WM]
     void* d_in = nullptr;       // host-input staging on the device
     float* d_outbuf = nullptr;  // host-output staging on the device
     // bicubic sweep: frames as float, 2-point gradients, 2x gradients, unit-gradient field
@@ -287,13 +288,14 @@ esrrf_status Shard::enqueue(const void* frames, int is_u16, float* out, float* h
             a.t0 = 0;
             a.int_weighting = int_weighting;
             a.cg_out = d_cg;
+            a.edge = d_edge;
             if (drift) {
                 SK(fht_drift_tables_build(m.geo[e], m.d_shift, m.d_shift + T, T, dtab, stream), "drift tables");
                 SK(fht_rgc_fused_drift(m.geo[e], dtab, a, stream), "RGC");
                 launches += 2;
             } else {
+                launches += fht_pair_pays(m.geo[e], m.tables[e], a) ? 2 : 1;
                 SK(fht_rgc_fused(m.geo[e], m.tables[e], a, stream), "RGC");
-                ++launches;
             }
             float* base = out + offsets[oi];
             for (int s0 = 0; s0 < (int)sens.size(); s0 += kSG)
@@ -417,6 +419,8 @@ void Shard::release() {
     scratch = InterpScratch();
     cudaFree(d_interp);
     cudaFree(d_cg);
+    cudaFree(d_edge);
+    d_edge = nullptr;
     cudaFree(d_in);
     cudaFree(d_outbuf);
     d_interp = d_cg = d_outbuf = nullptr;
@@ -551,6 +555,18 @@ esrrf_status Shard::create(const std::vector<float>& radii, int interp) {
         (e = cudaMalloc(&d_interp, sizeof(float) * (size_t)T * maxP)) != cudaSuccess ||
         (e = cudaMalloc(&d_cg, sizeof(float) * (size_t)T * maxP)) != cudaSuccess)
         return fail_cuda(e, "sweep buffers");
+    if (!drift) {
+        // the paired-tap kernel's second plane, where it leaves room for the staging of a host run;
+        // without it the fused kernel runs
+        const size_t want = sizeof(float) * (size_t)T * maxP;
+        const size_t later = sizeof(float) * (total + (size_t)T * w * h) + (size_t(256) << 20);
+        size_t avail = 0, all = 0;
+        if (cudaMemGetInfo(&avail, &all) != cudaSuccess || avail < want + later ||
+            cudaMalloc(&d_edge, want) != cudaSuccess) {
+            cudaGetLastError();
+            d_edge = nullptr;
+        }
+    }
     if (drift && (e = fht_drift_tables_alloc(maxS, T, maxP, dtab)) != cudaSuccess) return fail_cuda(e, "drift tables");
     if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return fail_cuda(e, "sync");
     return ESRRF_OK;
