@@ -408,12 +408,12 @@ def run_reference(args, world, rank):
     print(json.dumps(line))
 
 
-TRAFFIC_SUMMARIES = {"rgc_fused_fht512": "rgc_pair_fht512.md", "rgc_fused_bic512": "rgc_bic_bic512.md",
+TRAFFIC_SUMMARIES = {"rgc_fused_fht512": "rgc_pair_fht512.md", "rgc_fused_bic512": "bic_pair_bic512.md",
                      "rgc_fused_fht512_drift": "rgc_fused_drift_fht512.md"}
 # the kernel sources each summary's counts depend on
 SUMMARY_SOURCES = {
     "rgc_fused_fht512": ["rgc_pair.cuh"],
-    "rgc_fused_bic512": ["rgc_bic.cu", "device_common.cuh"],
+    "rgc_fused_bic512": ["bic_pair.cuh"],
     "rgc_fused_fht512_drift": ["fht_fused.cuh", "rgc_fht_drift.cu"],
 }
 
@@ -771,7 +771,7 @@ def run_ours(args, world, rank, local):
         "roofline": {"bound": "hbm", "achieved": achieved_gbs, "peak": peaks["hbm_gbs"],
                      "unit": "GB/s", "frac": achieved_gbs / peaks["hbm_gbs"],
                      "traffic": traffic, "peak_source": peak_src,
-                     "kernel": ("bic_rgc" if bic else "fht_rgc_pair" if args.kernel == "fused" and not args.drift
+                     "kernel": (("bic_pair" if args.kernel == "fused" else "bic_rgc") if bic else "fht_rgc_pair" if args.kernel == "fused" and not args.drift
                                 else f"fht_rgc_{args.kernel}"),
                      "avg_launch_ms": avg_launch_s * 1e3,
                      "alg_bytes_per_launch": alg_bytes_launch},

@@ -249,6 +249,21 @@ esrrf_status esrrf_handle::init_bic3d() {
         if (tbic_built) {
             CK(cudaMalloc(&d_u2, sizeof(float2) * bic_field_float2s(tbic, F)));
             CK(cudaMemsetAsync(d_u2, 0, sizeof(float2) * bic_field_float2s(tbic, F), stream));  // zero halo
+            CK(bic_pair_tables(bgeo, M, tpair));
+            const size_t px = (size_t)F * WM * HM;
+            if (!bic_pair_fits(tpair, ws, hs, M) || p.kernel != 0 ||
+                cudaMalloc(&d_nodes, sizeof(float2) * F * 4 * plane) != cudaSuccess ||
+                cudaMalloc(&d_own, sizeof(float) * px) != cudaSuccess ||
+                cudaMalloc(&d_edge, sizeof(float) * px) != cudaSuccess) {
+                // no such tables, or no room for its planes: the tabulated kernel takes every launch
+                cudaGetLastError();
+                bic_pair_tables_free(tpair);
+                cudaFree(d_nodes);
+                cudaFree(d_own);
+                cudaFree(d_edge);
+                d_nodes = nullptr;
+                d_own = d_edge = nullptr;
+            }
         }
     }
     CK(cudaMalloc(&d_mpmap, sizeof(float) * 3 * M * M * M));
@@ -323,6 +338,10 @@ void esrrf_handle::release() {
     cudaFree(d_u3);
     bic_tables_free(tbic);
     cudaFree(d_u2);
+    bic_pair_tables_free(tpair);
+    cudaFree(d_nodes);
+    cudaFree(d_own);
+    cudaFree(d_edge);
     for (float* b : {d_fraw, d_planes, d_gz, d_gxi, d_gyi, d_gzi, d_mpmap, mfm.coeff, mfm.cos_t,
                      mfm.sin_t, mfm.shx, mfm.shy})
         cudaFree(b);
@@ -476,7 +495,15 @@ esrrf_status esrrf_handle::process_chunk_bic3d(const void* src, bool is_u16, int
             return r;
         CK(cudaEventRecord(e0, stream));
     }
-    if (mode == Mode::kBIC) {
+    // tabulated taps unless a frame of this launch has drift or the plain kernel was asked for
+    bool no_drift = p.kernel == 0;
+    for (int i = 0; i < 2 * F_now; ++i) no_drift = no_drift && sh[i] == 0.f;
+    const bool paired = mode == Mode::kBIC && no_drift && bic_pair_pays(tpair, ws, hs, p.magnification, F_now);
+    grad_stale = paired;
+    if (paired) {
+        CK(bic_nodes(src, is_u16 ? 1 : 0, ws, hs, F_now, d_fraw, d_nodes, stream));
+        launches += 1;
+    } else if (mode == Mode::kBIC) {
         CK(bic_prepare(src, is_u16 ? 1 : 0, W, H, F_now, d_fraw, d_gx, d_gy, d_gxi, d_gyi, stream));
         launches += 3;
     } else {
@@ -485,10 +512,24 @@ esrrf_status esrrf_handle::process_chunk_bic3d(const void* src, bool is_u16, int
         launches += 6;
     }
     if (timing) CK(cudaEventRecord(e1, stream));
-    // tabulated taps unless a frame of this launch has drift or the plain kernel was asked for
-    bool no_drift = p.kernel == 0;
-    for (int i = 0; i < 2 * F_now; ++i) no_drift = no_drift && sh[i] == 0.f;
-    if (mode == Mode::kBIC && no_drift && tbic_built) {
+    if (paired) {
+        BicPairRun r{};
+        r.U = d_nodes;
+        r.fraw = d_fraw;
+        r.wsum = tbic.wsum;
+        r.own = d_own;
+        r.edge = d_edge;
+        r.w = ws;
+        r.h = hs;
+        r.M = p.magnification;
+        r.F = F_now;
+        r.t0 = frame_in_block;
+        r.sens = bgeo.sensitivity;
+        r.int_weighting = p.int_weighting;
+        r.st = st;
+        CK(bic_rgc_pair(r, tpair, stream));
+        launches += 1;
+    } else if (mode == Mode::kBIC && no_drift && tbic_built) {
         CK(unit_grad2d(d_gxi, d_gyi, ws, hs, F_now, tbic, d_u2, stream));
         BicTabArgs ta{};
         ta.U = d_u2;
@@ -864,6 +905,13 @@ esrrf_status esrrf_read_gradients(esrrf_handle* h, float* out, size_t out_len) {
     if (h->mode != esrrf_handle::Mode::kFHT) {
         // 2x-resampled gradient components of the first frame of the last push
         const size_t plane = (size_t)4 * h->ws * h->hs * h->P;
+        // the paired form leaves no gradient planes: those of the first frame, from its float copy
+        if (h->grad_stale &&
+            bic_prepare(h->d_fraw, 0, h->ws, h->hs, 1, (float*)h->d_nodes, h->d_gx, h->d_gy, h->d_gxi, h->d_gyi, h->stream) !=
+                cudaSuccess) {
+            cudaGetLastError();
+            return h->fail(ESRRF_ERR_CUDA, "gradient read-back failed");
+        }
         const int nc = h->mode == esrrf_handle::Mode::k3D ? 3 : 2;
         if (out_len < nc * plane) return h->fail(ESRRF_ERR_INVALID, "output buffer too small");
         const float* src[3] = {h->d_gxi, h->d_gyi, h->d_gzi};

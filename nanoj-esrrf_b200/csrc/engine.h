@@ -64,6 +64,11 @@ struct esrrf_handle {
     esrrf::BicTables tbic;      // 2-D bicubic tap tables per sub-pixel phase (launches without drift)
     bool tbic_built = false;
     float2* d_u2 = nullptr;     // [F][2hs][2ws] padded unit gradient field (2-D bicubic)
+    esrrf::BicPairTables tpair; // paired-tap form of the bicubic RGC (null where it does not apply)
+    float2* d_nodes = nullptr;  // [F][2hs][2ws] unit gradient at the nodes, for it
+    float* d_own = nullptr;     // [F][HM][WM] its two planes
+    float* d_edge = nullptr;
+    bool grad_stale = false;    // bicubic: the last push took the paired form, which leaves no gradient planes
 
     // input staging (double-buffered)
     size_t raw_frame_bytes = 0;

@@ -279,6 +279,35 @@ struct BicTabArgs {
 cudaError_t unit_grad2d(const float* gxi, const float* gyi, int w, int h, int F, const BicTables& t,
                         float2* U, cudaStream_t stream);
 cudaError_t bic_rgc_tab(const BicTabArgs& a, cudaStream_t stream);
+// Paired-tap form of the bicubic RGC (bic_pair.cuh) for launches without drift at magnifications 2 and
+// 4 whose discs reach at most 15 output pixels.
+struct BicPairTables {
+    float2* wt = nullptr;  // device [I + 1][16] (w, w / d in output pixels)
+    int I = 0;             // largest column distance
+    int taps = 0;          // taps of an output pixel
+    signed char J[16] = {};
+};
+cudaError_t bic_pair_tables(const BicGeometry& g, int M, BicPairTables& t);  // t.wt null: not supported
+void bic_pair_tables_free(BicPairTables& t);
+bool bic_pair_fits(const BicPairTables& t, int w, int h, int M);
+// Whether it is the faster form for a launch of F frames.
+bool bic_pair_pays(const BicPairTables& t, int w, int h, int M, int F);
+// raw -> float frames and the unit gradient at the nodes [F][2h][2w]
+cudaError_t bic_nodes(const void* raw, int is_u16, int w, int h, int F, float* fraw, float2* U, cudaStream_t stream);
+struct BicPairRun {
+    const float2* U;
+    const float* fraw;
+    const float* wsum;   // [hM][wM] (BicTables::wsum)
+    float* own;          // [F][hM][wM] scratch planes (per-frame mode: cg_out in the place of own)
+    float* edge;
+    int w, h, M, F, t0;
+    float sens;
+    int int_weighting;
+    BlockState st;
+    float* cg_out;       // per-frame mode (the sweep): CGLH / sum of weights and the intensity
+    float* v_out;
+};
+cudaError_t bic_rgc_pair(const BicPairRun& r, const BicPairTables& t, cudaStream_t stream);
 // MP map of AVG/VAR/TAC2 and division (then NaN->0) on a finalized output [4][PM][HM][WM].
 cudaError_t mp_correct(float* out, int w, int h, int P, int M, int is3d, float* map,
                        cudaStream_t stream);

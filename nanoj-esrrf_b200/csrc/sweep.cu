@@ -154,6 +154,7 @@ struct MagPlan {
     std::vector<FhtFusedTables> tables; // per entry of ri
     std::vector<BicGeometry> bgeo;      // bicubic sweep: per entry of ri
     std::vector<BicTables> btab;        // bicubic sweep: per entry of ri (common field padding)
+    std::vector<BicPairTables> bpair;   // and its paired-tap form (no weights: the tabulated kernel runs)
     float* d_shift = nullptr;           // drift x M, [2][T] (FHT sweep with drift)
 };
 
@@ -176,7 +177,7 @@ struct Shard {
     InterpScratch scratch;
     float* d_interp = nullptr;  // [T][HM][WM] for the largest magnification
     float* d_cg = nullptr;
-    float* d_edge = nullptr;    // FHT sweep without drift: the paired-tap kernel's second plane [T][HM][WM]
+    float* d_edge = nullptr;    // the paired-tap kernels' second plane [T][HM][WM]
     void* d_in = nullptr;       // host-input staging on the device
     float* d_outbuf = nullptr;  // host-output staging on the device
     // bicubic sweep: frames as float, 2-point gradients, 2x gradients, unit-gradient field
@@ -187,6 +188,8 @@ struct Shard {
     float* d_gxi = nullptr;
     float* d_gyi = nullptr;
     float2* d_u2 = nullptr;
+    float2* d_nodes = nullptr;  // unit gradient at the nodes (entries with a paired-tap form)
+    bool tabulated = false;     // some entry runs the tabulated kernel
     float* d_mpmap = nullptr;
     std::vector<size_t> offsets;  // local layout: per (mp entry, radius entry) in order
     size_t total = 0;
@@ -331,30 +334,54 @@ esrrf_status Shard::enqueue(const void* frames, int is_u16, float* out, float* h
 esrrf_status Shard::enqueue_bic(const void* frames, int is_u16, float* out, float* hout) {
     Shard* s = this;
     int launches = 0;
-    SK(bic_prepare(frames, is_u16, w, h, T, d_fraw, d_gx, d_gy, d_gxi, d_gyi, stream), "gradients");
-    launches += 3;
-    SK(unit_grad2d(d_gxi, d_gyi, w, h, T, mp[0].btab[0], d_u2, stream), "unit gradient");
-    ++launches;
+    if (tabulated) {
+        SK(bic_prepare(frames, is_u16, w, h, T, d_fraw, d_gx, d_gy, d_gxi, d_gyi, stream), "gradients");
+        launches += 3;
+        SK(unit_grad2d(d_gxi, d_gyi, w, h, T, mp[0].btab[0], d_u2, stream), "unit gradient");
+        ++launches;
+    }
+    if (d_nodes) {
+        SK(bic_nodes(frames, is_u16, w, h, T, d_fraw, d_nodes, stream), "gradients");
+        ++launches;
+    }
     size_t oi = 0;
     for (size_t mi = 0; mi < mp.size(); ++mi) {
         const MagPlan& m = mp[mi];
         const long P = (long)w * m.M * h * m.M;
         for (size_t e = 0; e < m.ri.size(); ++e, ++oi) {
-            BicTabArgs a{};
-            a.U = d_u2;
-            a.fraw = d_fraw;
-            a.w = w;
-            a.h = h;
-            a.M = m.M;
-            a.F = T;
-            a.t0 = 0;
-            a.sens = 1.f;
-            a.int_weighting = int_weighting;
-            a.tab = m.btab[e];
-            a.cg_out = d_cg;
-            a.v_out = d_interp;
-            SK(bic_rgc_tab(a, stream), "RGC");
-            ++launches;
+            if (m.bpair[e].wt) {
+                BicPairRun r{};
+                r.U = d_nodes;
+                r.fraw = d_fraw;
+                r.wsum = m.btab[e].wsum;
+                r.edge = d_edge;
+                r.w = w;
+                r.h = h;
+                r.M = m.M;
+                r.F = T;
+                r.sens = 1.f;
+                r.int_weighting = int_weighting;
+                r.cg_out = d_cg;
+                r.v_out = d_interp;
+                SK(bic_rgc_pair(r, m.bpair[e], stream), "RGC");
+                launches += 2;
+            } else {
+                BicTabArgs a{};
+                a.U = d_u2;
+                a.fraw = d_fraw;
+                a.w = w;
+                a.h = h;
+                a.M = m.M;
+                a.F = T;
+                a.t0 = 0;
+                a.sens = 1.f;
+                a.int_weighting = int_weighting;
+                a.tab = m.btab[e];
+                a.cg_out = d_cg;
+                a.v_out = d_interp;
+                SK(bic_rgc_tab(a, stream), "RGC");
+                ++launches;
+            }
             float* base = out + offsets[oi];
             for (int s0 = 0; s0 < (int)sens.size(); s0 += kSG)
                 for (int b0 = 0; b0 < (int)bstart.size(); b0 += kBG) {
@@ -404,11 +431,14 @@ void Shard::release() {
         interp_plan_destroy(m.plan);
         for (auto& t : m.tables) fht_fused_tables_free(t);
         for (auto& t : m.btab) bic_tables_free(t);
+        for (auto& t : m.bpair) bic_pair_tables_free(t);
         cudaFree(m.d_shift);
     }
     fht_drift_tables_free(dtab);
     for (float* b : {d_fraw, d_gx, d_gy, d_gxi, d_gyi, d_mpmap}) cudaFree(b);
     cudaFree(d_u2);
+    cudaFree(d_nodes);
+    d_nodes = nullptr;
     d_fraw = d_gx = d_gy = d_gxi = d_gyi = d_mpmap = nullptr;
     d_u2 = nullptr;
     mp.clear();
@@ -491,6 +521,33 @@ esrrf_status Shard::create_bic(const std::vector<float>& radii) {
         return fail_cuda(e, "sweep buffers");
     if ((e = cudaMemsetAsync(d_u2, 0, sizeof(float2) * field, stream)) != cudaSuccess)  // zero halo
         return fail_cuda(e, "sweep buffers");
+    // paired-tap forms where they are the faster ones and their planes leave room for the staging of a
+    // host run
+    bool some = false;
+    for (auto& m : mp)
+        for (size_t i = 0; i < m.ri.size(); ++i) {
+            BicPairTables t;
+            if ((e = bic_pair_tables(m.bgeo[i], m.M, t)) != cudaSuccess) return fail_cuda(e, "RGC tables");
+            if (!bic_pair_fits(t, w, h, m.M) || !bic_pair_pays(t, w, h, m.M, T)) bic_pair_tables_free(t);
+            some = some || t.wt;
+            m.bpair.push_back(t);
+        }
+    if (some) {
+        const size_t edge = sizeof(float) * (size_t)T * maxP, nodes = sizeof(float2) * (size_t)T * 4 * plane;
+        const size_t later = sizeof(float) * (total + (size_t)T * plane) + (size_t(256) << 20);
+        size_t avail = 0, all = 0;
+        if (cudaMemGetInfo(&avail, &all) != cudaSuccess || avail < edge + nodes + later ||
+            cudaMalloc(&d_edge, edge) != cudaSuccess || cudaMalloc(&d_nodes, nodes) != cudaSuccess) {
+            cudaGetLastError();
+            cudaFree(d_edge);
+            d_edge = nullptr;
+            d_nodes = nullptr;
+            for (auto& m : mp)
+                for (auto& t : m.bpair) bic_pair_tables_free(t);
+        }
+    }
+    for (auto& m : mp)
+        for (auto& t : m.bpair) tabulated = tabulated || !t.wt;
     if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return fail_cuda(e, "sync");
     return ESRRF_OK;
 }
