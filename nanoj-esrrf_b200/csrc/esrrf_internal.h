@@ -45,6 +45,8 @@ struct InterpPlan {
     bool tc = false;
     float* dxp = nullptr;     // pass 1 B panels [WM/256][N/16] (hi, lo)
     float* dyp = nullptr;     // pass 2 A panels [HM/128][N/16] (hi, lo)
+    int* quads = nullptr;     // pass 1's stores: padded rows in fours by the rows that they repeat
+    int quads_once = 0;       // offset in quads of the table for the h frame rows
     int* tc_err = nullptr;
 };
 
@@ -71,7 +73,8 @@ cudaError_t interp_adjoint_run(const InterpPlan& p, const float* dx, const float
 // Tensor-core (tcgen05, three-term TF32) form of the two dense passes; needs N % 128 == 0.
 // Writes the first-pass rows into scratch.rowT as pass 2's operand panels.
 bool tc_interp_supported(const InterpPlan& plan);
-cudaError_t tc_plan_tables(InterpPlan& plan, const std::vector<float>& dxT, const std::vector<float>& dy);
+cudaError_t tc_plan_tables(InterpPlan& plan, const std::vector<float>& dxT, const std::vector<float>& dy,
+                           const std::vector<int>& srcy);
 // Scratch floats per frame: first-pass rows (either form) and the frame's operand panels.
 size_t interp_rowT_floats(const InterpPlan& plan);
 size_t interp_xs_floats(const InterpPlan& plan);

@@ -561,7 +561,7 @@ cudaError_t interp_plan_create(InterpPlan& p, int w, int h, int M, int scale_mod
     if ((e = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev)) != cudaSuccess)
         return e;
     p.tc = major == 10 && tc_interp_supported(p) && !(sel && std::strcmp(sel, "simt") == 0);
-    if (p.tc) return tc_plan_tables(p, dxT, dy);
+    if (p.tc) return tc_plan_tables(p, dxT, dy, sy);
     return cudaSuccess;
 }
 
@@ -577,6 +577,7 @@ void interp_plan_destroy(InterpPlan& p) {
     cudaFree(p.srcy);
     cudaFree(p.dxp);
     cudaFree(p.dyp);
+    cudaFree(p.quads);
     cudaFree(p.tc_err);
     p = InterpPlan();
 }

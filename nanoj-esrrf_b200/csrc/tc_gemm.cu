@@ -6,11 +6,16 @@
 //   pass 1:  rowsT[f] (WM x N)  = (X_f - c_f) Dx^T, written split into pass 2's operand panels
 //   pass 2:  I'[f]    (HM x WM) = Dy rowsT[f]^T + rank-one terms + c_f s N^2
 //
+// The N x N padded frame repeats the frame's rows mirrored, so a large launch's pass 1 contracts each of the
+// h rows once and its epilogue writes the result at every padded row that repeats it (TcArgs::quads): the same sums in
+// the same order as over all N rows.  100 frames of 640 x 360 (N = 1024) at M2 with the rest of their block:
+// 4.19 ms with pass 1 over all rows, 3.30 ms with each row once.
+//
 // Operands live in HBM already split and laid out as "panels": for a tile of R rows (128 for A,
 // 256 for B) and a K block of 16, the hi part then the lo part, each in the canonical K-major
 // no-swizzle core-matrix layout (core matrix = 8 rows x 16 bytes; the 16-byte chunk k4 of row r
 // at ((k4 (R/8) + r/8) 128 + (r%8) 16) bytes).  Dx and Dy panels are built once per plan, the
-// padded frame's panels by x_split_kernel, and pass 1's epilogue writes pass 2's B panels.  So a
+// frame's panels by x_split_kernel, and pass 1's epilogue writes pass 2's B panels.  So a
 // pipeline stage is filled by two plain bulk copies (cp.async.bulk, no tensor map, no multicast).
 //
 // CTA: 10 warps.  Warp 8 (one lane) streams the panels into a ring of 4 shared-memory stages of
@@ -46,6 +51,7 @@ constexpr uint32_t TC_SMEM_BYTES = TC_STAGES * TC_STAGE;
 constexpr int TC_RUN = 2;                 // K blocks per accumulator run (K = 32)
 constexpr uint32_t TC_TMEM_COLS = 512;    // two 128 x 256 FP32 accumulators
 constexpr int TC_THREADS = 320;
+constexpr int TC_ST = 20;  // floats between rows of a warp's store stage
 constexpr long long TC_WAIT_CYCLES = 4000000000LL;  // ~2 s of SM clock before a wait gives up
 
 // Instruction descriptor: D f32 (bits 4-5 = 1), A tf32 (7-9 = 2), B tf32 (10-12 = 2), both
@@ -154,9 +160,12 @@ struct TcArgs {
     long a_frame;                    // bytes between frames' A panels (0: shared)
     const unsigned char* Bp;         // B panels [nt][kb], TC_B_BYTES each
     long b_frame;
-    // pass 1: C written as pass 2's B panels [f][nt][kb2] (K of pass 2 = the rows here)
+    // pass 1: C written as pass 2's B panels [f][nt][kb2] (K of pass 2 = the padded rows, nkb2 blocks of
+    // 16), each row at all padded rows that repeat it (quads)
     unsigned char* Cp;
     long c_frame;
+    int nkb2;
+    const int* quads;
     // pass 2: C row-major [f][Mr][Nc] plus the rank-one terms
     float* C;
     const float* vec;
@@ -170,12 +179,65 @@ struct TcArgs {
     int* err;
 };
 
+// Pass 1's epilogue for one warp: its 32 rows x 128 columns (C^T: the columns are pass 2's output columns,
+// the rows its K), split, into pass 2's B panels.  16 columns at a time go through the warp's stage,
+// so that a lane writes one column's four consecutive padded rows (a quad: 16 bytes of a panel) and a
+// half warp 256 contiguous bytes, where one float per lane and store, straight from the accumulators,
+// touches eight lines an instruction.  The quads that hold a row of the warp come from the plan, with the
+// row in the warp of each of the four (255: a row of another warp).
+__device__ __forceinline__ void store_rows(const TcArgs& g, const float* racc, float* st, int r0, int c0, int nt,
+                                           int f, int lane) {
+    if (r0 >= g.Mr) return;
+    const int* start = g.quads;
+    const int2* quad = reinterpret_cast<const int2*>(g.quads + start[0]);
+    const int first = start[1 + r0 / 32] + (lane >> 4), end = start[2 + r0 / 32];
+    unsigned char* Cf = g.Cp + (long)f * g.c_frame + (long)nt * g.nkb2 * TC_B_BYTES;
+    const int col = lane & 15;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            *reinterpret_cast<float4*>(st + lane * TC_ST + 4 * j) = make_float4(
+                racc[16 * c + 4 * j], racc[16 * c + 4 * j + 1], racc[16 * c + 4 * j + 2], racc[16 * c + 4 * j + 3]);
+        __syncwarp();
+        if (c0 + 16 * c + col >= g.Nc) continue;
+        const int rr = ((c0 + 16 * c) & (TC_N - 1)) + col;
+#pragma unroll 1
+        for (int q = first; q < end; q += 2) {
+            const int2 e = __ldg(quad + q);  // padded rows 4 e.x .. 4 e.x + 3
+            unsigned char* P = Cf + (long)(e.x >> 2) * TC_B_BYTES + panel_off(TC_N, rr, e.x & 3);
+            float4 hi, lo;
+            float* hp = &hi.x;
+            float* lp = &lo.x;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float v = st[((e.y >> (8 * i)) & 31) * TC_ST + col];
+                hp[i] = tf32_rna(v);
+                lp[i] = tf32_rna(v - hp[i]);
+            }
+            if ((e.y & 0x80808080) == 0) {
+                *reinterpret_cast<float4*>(P) = hi;
+                *reinterpret_cast<float4*>(P + TC_B_PANEL) = lo;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (((e.y >> (8 * i)) & 128) == 0) {
+                        reinterpret_cast<float*>(P)[i] = hp[i];
+                        reinterpret_cast<float*>(P + TC_B_PANEL)[i] = lp[i];
+                    }
+            }
+        }
+    }
+}
+
 template <int PASS>
 __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(TcArgs g) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ __align__(8) uint64_t bar_full[TC_STAGES], bar_empty[TC_STAGES], bar_accf[2], bar_acce[2];
     __shared__ uint32_t tmem_slot;
     __shared__ __align__(16) float4 colterm[TC_N];  // pass 2: (cx, ux, q, r) of the tile's columns
+    __shared__ __align__(16) float stage[PASS == 1 ? 8 : 1][32 * TC_ST];  // pass 1: a warp's rows, 16 columns
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int f = blockIdx.z, mt = blockIdx.y, nt = blockIdx.x;
     const int m0 = mt * TC_M, n0 = nt * TC_N;
@@ -317,22 +379,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_kernel(TcArgs g) {
         const int row = m0 + 32 * (warp & 3) + lane;
         const int cb = (warp >> 2) * 128;  // column offset within the tile
         if (PASS == 1) {
-            // C^T (columns n = output columns of pass 2, rows = K of pass 2) into pass 2's B
-            // panels, split: panel (nt, kb2 = row / 16), panel row n - n0, k = row % 16
-            if (row < g.Mr) {
-                unsigned char* P = g.Cp + (long)f * g.c_frame +
-                                   ((long)nt * (g.Mr / TC_BK) + row / TC_BK) * TC_B_BYTES;
-                const int k = row % TC_BK;
-#pragma unroll
-                for (int j = 0; j < 128; ++j) {
-                    const int rr = cb + j;
-                    if (n0 + rr >= g.Nc) break;
-                    const uint32_t off = panel_off(TC_N, rr, k >> 2) + ((k & 3) << 2);
-                    const float hi = tf32_rna(racc[j]);
-                    *reinterpret_cast<float*>(P + off) = hi;
-                    *reinterpret_cast<float*>(P + TC_B_PANEL + off) = tf32_rna(racc[j] - hi);
-                }
-            }
+            store_rows(g, racc, stage[warp], m0 + 32 * (warp & 3), n0 + cb, nt, f, lane);
         } else {
             if (row < g.Mr) {
                 const float* vec = g.vec + (long)f * (2L * g.HM + 2L * g.WM + 1);
@@ -385,6 +432,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_pkernel(TcArgs g, int n
     __shared__ __align__(8) uint64_t bar_full[TC_STAGES], bar_empty[TC_STAGES], bar_accf[2], bar_acce[2];
     __shared__ uint32_t tmem_slot;
     __shared__ __align__(16) float4 colterm[TC_N];  // pass 2: (cx, ux, q, r) of the tile's columns
+    __shared__ __align__(16) float stage[PASS == 1 ? 8 : 1][32 * TC_ST];  // pass 1: a warp's rows, 16 columns
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nkb = g.nkb, nruns = (nkb + TC_RUN - 1) / TC_RUN;
     const int T = ntx * nty * nframes;
@@ -538,20 +586,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_pkernel(TcArgs g, int n
             const int row = m0 + 32 * (warp & 3) + lane;
             const int cb = (warp >> 2) * 128;
             if (PASS == 1) {
-                if (row < g.Mr) {
-                    unsigned char* P = g.Cp + (long)f * g.c_frame +
-                                       ((long)nt * (g.Mr / TC_BK) + row / TC_BK) * TC_B_BYTES;
-                    const int k = row % TC_BK;
-#pragma unroll
-                    for (int j = 0; j < 128; ++j) {
-                        const int rr = cb + j;
-                        if (n0 + rr >= g.Nc) break;
-                        const uint32_t off = panel_off(TC_N, rr, k >> 2) + ((k & 3) << 2);
-                        const float hi = tf32_rna(racc[j]);
-                        *reinterpret_cast<float*>(P + off) = hi;
-                        *reinterpret_cast<float*>(P + TC_B_PANEL + off) = tf32_rna(racc[j] - hi);
-                    }
-                }
+                store_rows(g, racc, stage[warp], m0 + 32 * (warp & 3), n0 + cb, nt, f, lane);
             } else if (row < g.Mr) {
                 const float* vec = g.vec + (long)f * (2L * g.HM + 2L * g.WM + 1);
                 const float pm = vec[row], tm = vec[g.HM + row];
@@ -591,17 +626,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm_pkernel(TcArgs g, int n
     }
 }
 
-// Padded frame minus its mean, split into pass 1's A panels [f][mt][kb].  One thread per 16-byte
-// chunk; consecutive threads take consecutive rows of one chunk column (coalesced panel writes).
+// The frame's rows (srcy: the padded frame's), padded along x, minus the mean, split into pass 1's A panels
+// [f][mt][kb] (zero rows beyond the frame's in the last tile).  One thread per 16-byte chunk; consecutive threads take consecutive rows of one chunk column (coalesced panel writes).
 __global__ void __launch_bounds__(256) x_split_kernel(const void* __restrict__ raw, int is_u16, int w, int h,
-                                                      int N, const int* __restrict__ srcx,
+                                                      int N, long nchunks, const int* __restrict__ srcx,
                                                       const int* __restrict__ srcy,
                                                       const float* __restrict__ vec, long vstride,
                                                       long cmean_off, unsigned char* __restrict__ xp) {
     const int f = blockIdx.y;
     const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;  // chunk index in the frame
     const long per_panel = TC_M * (TC_BK / 4);
-    const long nchunks = (long)N * N / 4;
     if (q >= nchunks) return;
     const long p = q / per_panel;
     const int within = (int)(q - p * per_panel);
@@ -610,7 +644,7 @@ __global__ void __launch_bounds__(256) x_split_kernel(const void* __restrict__ r
     const int mt = (int)(p / nkb), kb = (int)(p % nkb);
     const int m = mt * TC_M + r, x = kb * TC_BK + 4 * k4;
     const float c = vec[(long)f * vstride + cmean_off];
-    const long row = (long)srcy[m] * w + (long)f * w * h;
+    const long row = (long)(srcy ? srcy[m] : min(m, h - 1)) * w + (long)f * w * h;
     const int4 sx = *reinterpret_cast<const int4*>(srcx + x);
     float v[4];
     if (is_u16) {
@@ -625,11 +659,11 @@ __global__ void __launch_bounds__(256) x_split_kernel(const void* __restrict__ r
     float* lp = &lo.x;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const float d = v[i] - c;
+        const float d = srcy || m < h ? v[i] - c : 0.f;
         hp[i] = tf32_rna(d);
         lp[i] = tf32_rna(d - hp[i]);
     }
-    unsigned char* P = xp + ((long)f * (N / TC_M) * nkb + p) * TC_A_BYTES;
+    unsigned char* P = xp + ((long)f * (nchunks / per_panel) + p) * TC_A_BYTES;
     const uint32_t off = panel_off(TC_M, r, k4);
     *reinterpret_cast<float4*>(P + off) = hi;
     *reinterpret_cast<float4*>(P + TC_A_PANEL + off) = lo;
@@ -705,8 +739,35 @@ size_t interp_rowT_floats(const InterpPlan& p) {
 
 size_t interp_xs_floats(const InterpPlan& p) { return p.tc ? (size_t)p.N * p.N * 2 : 0; }
 
-cudaError_t tc_plan_tables(InterpPlan& p, const std::vector<float>& dxT, const std::vector<float>& dy) {
-    const int N = p.N;
+cudaError_t tc_plan_tables(InterpPlan& p, const std::vector<float>& dxT, const std::vector<float>& dy,
+                           const std::vector<int>& srcy) {
+    const int N = p.N, h = p.h;
+    // quads of padded rows by the 32 rows that they repeat, for the N padded rows themselves and then for
+    // the h frame rows (quads_once): [0] the offset of the quads (even, for 8-byte loads), [1 + i] the
+    // first of rows 32 i .., then (quad, the four rows of the 32, or 255)
+    std::vector<int> quads;
+    for (const bool once : {false, true}) {
+        const int groups = ((once ? h : N) + 31) / 32;
+        std::vector<int> head((groups + 3) & ~1, 0), body;
+        head[0] = (int)head.size();
+        for (int i = 0; i < groups; ++i) {
+            for (int m = 0; m < N; m += 4) {
+                unsigned rows = 0;
+                for (int k = 0; k < 4; ++k) {
+                    const int r = once ? srcy[m + k] : m + k;
+                    rows |= (r / 32 == i ? (unsigned)(r % 32) : 255u) << (8 * k);
+                }
+                if (rows != 0xffffffffu) {
+                    body.push_back(m / 4);
+                    body.push_back((int)rows);
+                }
+            }
+            head[2 + i] = (int)body.size() / 2;
+        }
+        if (once) p.quads_once = (int)quads.size();
+        quads.insert(quads.end(), head.begin(), head.end());
+        quads.insert(quads.end(), body.begin(), body.end());
+    }
     std::vector<float> dx((size_t)p.WM * N);
     for (int n = 0; n < p.WM; ++n)
         for (int m = 0; m < N; ++m) dx[(size_t)n * N + m] = dxT[(size_t)m * p.WM + n];
@@ -718,6 +779,9 @@ cudaError_t tc_plan_tables(InterpPlan& p, const std::vector<float>& dxT, const s
         return e;
     if ((e = cudaMalloc((void**)&p.dyp, sizeof(float) * dyp.size())) != cudaSuccess) return e;
     if ((e = cudaMemcpy(p.dyp, dyp.data(), sizeof(float) * dyp.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
+        return e;
+    if ((e = cudaMalloc((void**)&p.quads, sizeof(int) * quads.size())) != cudaSuccess) return e;
+    if ((e = cudaMemcpy(p.quads, quads.data(), sizeof(int) * quads.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
         return e;
     if ((e = cudaMalloc((void**)&p.tc_err, sizeof(int))) != cudaSuccess) return e;
     return cudaMemset(p.tc_err, 0, sizeof(int));
@@ -743,11 +807,20 @@ cudaError_t tc_interp_passes(const InterpPlan& p, InterpScratch& sc, const void*
     if ((e = set_tc_smem<2>()) != cudaSuccess) return e;
     const int N = p.N, nkb = N / TC_BK;
     const int ntiles = (p.WM + TC_N - 1) / TC_N;
+    int dev = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    const int sms = sm_count(dev);
+    // Pass 1 over the h frame rows where the padded rows would give every SM two tiles or more, that
+    // leaves tiles out, and all four row warps of a tile have rows: a warp stores its rows' copies one
+    // after the other, which a launch of few tiles would wait for (one 300 x 110 frame at M2 with its
+    // analysis: 115 us over all rows, 146 us with each once; 60 frames of 900 x 100: 2.29 and 1.50 ms).
+    const bool once = p.h > 96 && (p.h + TC_M - 1) / TC_M < N / TC_M && (long)ntiles * (N / TC_M) * F >= 2L * sms;
+    const int rows = once ? p.h : N, mtiles1 = (rows + TC_M - 1) / TC_M;
     const long vstride = 2L * p.HM + 2L * p.WM + 1;
     {
-        const long chunks = (long)N * N / 4;
+        const long chunks = (long)mtiles1 * TC_M * N / 4;
         x_split_kernel<<<dim3((unsigned)((chunks + 255) / 256), F), 256, 0, stream>>>(
-            raw, is_u16 ? 1 : 0, p.w, p.h, N, p.srcx, p.srcy, sc.vec, vstride, 2L * p.HM + 2L * p.WM,
+            raw, is_u16 ? 1 : 0, p.w, p.h, N, chunks, p.srcx, once ? nullptr : p.srcy, sc.vec, vstride, 2L * p.HM + 2L * p.WM,
             reinterpret_cast<unsigned char*>(sc.xs));
     }
     TcArgs g{};
@@ -762,25 +835,24 @@ cudaError_t tc_interp_passes(const InterpPlan& p, InterpScratch& sc, const void*
     g.err = p.tc_err;
     const long rowT_frame = (long)ntiles * nkb * TC_B_BYTES;
     // pass 1: rows of (X - c) times Dx^T, written as pass 2's B panels
-    g.Mr = N;
+    g.Mr = rows;
     g.Nc = p.WM;
     g.nkb = nkb;
     g.Ap = reinterpret_cast<const unsigned char*>(sc.xs);
-    g.a_frame = (long)(N / TC_M) * nkb * TC_A_BYTES;
+    g.a_frame = (long)mtiles1 * nkb * TC_A_BYTES;
     g.Bp = reinterpret_cast<const unsigned char*>(p.dxp);
     g.b_frame = 0;
     g.Cp = reinterpret_cast<unsigned char*>(sc.rowT);
     g.c_frame = rowT_frame;
-    int dev = 0;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    g.nkb2 = nkb;
+    g.quads = p.quads + (once ? p.quads_once : 0);
     const bool pers = tc_persistent();
-    const int sms = sm_count(dev);
     auto pgrid = [&](int tiles) { return (unsigned)std::max(1, std::min(tiles, sms)); };
     if (pers)
-        tc_gemm_pkernel<1><<<pgrid(ntiles * (N / TC_M) * F), TC_THREADS, TC_SMEM_BYTES, stream>>>(
-            g, ntiles, N / TC_M, F);
+        tc_gemm_pkernel<1><<<pgrid(ntiles * mtiles1 * F), TC_THREADS, TC_SMEM_BYTES, stream>>>(g, ntiles,
+                                                                                               mtiles1, F);
     else
-        tc_gemm_kernel<1><<<dim3(ntiles, N / TC_M, F), TC_THREADS, TC_SMEM_BYTES, stream>>>(g);
+        tc_gemm_kernel<1><<<dim3(ntiles, mtiles1, F), TC_THREADS, TC_SMEM_BYTES, stream>>>(g);
     // pass 2: Dy times the first-pass rows, plus the rank-one terms
     g.Mr = p.HM;
     g.Nc = p.WM;

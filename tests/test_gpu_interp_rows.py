@@ -1,0 +1,29 @@
+"""The tensor-core interpolation contracts each row of the frame once and writes the result at every
+padded row that mirrors it: frames whose padded square repeats a row many times, once or not at all, row
+counts around a tile of 128 and a K block of 16, against the float64 interpolation of the padded frame.
+Tolerance: 2e-6 of the slice's range, as for square frames (the sums are the same)."""
+import numpy as np
+import pytest
+
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("w,h,M", [(300, 20, 2), (9, 200, 3), (129, 127, 2), (255, 129, 4), (128, 40, 5), (65, 33, 4),
+                                   (256, 17, 2), (161, 144, 3), (128, 128, 2)])
+def test_rows_once(esrrf_mod, w, h, M):
+    from esrrf import synth
+    from oracle import adjoint_oracle as A
+    raw = synth.small_stack(200 + w + h + M, 2, h, w)
+    ref = A.interpolate_f64(raw.astype(np.float64), M).mean(axis=0)
+    for frames in (raw, raw.astype(np.float32)):
+        eng = esrrf_mod.LiveSRRF_CL()
+        eng.initialise(w, h, M, 1.0, 1, 2, 2)
+        try:
+            eng.resetFramePosition()
+            assert not eng.calculateSRRF(frames)
+            got = eng.readSRRFbuffer()[3].copy()
+        finally:
+            eng.release()
+        assert rel_err(got, ref) < 2e-6
