@@ -131,7 +131,9 @@ cudaError_t fht_pair_tables(const FhtGeometry& g, FhtFusedTables& t, cudaStream_
 // with segments up to 100 rows, 0.13 from 400 rows on (the widest boxes a fifth more), 34.7 us per tile
 // and frame for the fused kernel (0.67 of that where every SM has one tile at most; a tenth more
 // with several frame groups, which add into the sums with atomics).  On 56 launches from 48 x 48 to
-// 900 x 450 with boxes of 6 to 32 the rule takes the slower kernel only where they are within 5 %.
+// 900 x 450 with boxes of 6 to 32 the rule takes the slower kernel only where they are within 5 %;
+// for one frame the fused kernel stays unless the other is ahead by as much (221 x 163 at M4, box 10:
+// modelled 49.0 / 49.7 us, measured 5 us behind).
 // Paired against fused, one block: 100 frames of 512 x 512 at M4 15.1 / 24.7 ms, 10 of 128 x 128 161 /
 // 229 us, one of 256 x 256 103 / 96 us, one of 128 x 128 82 / 39 us.
 bool fht_pair_pays(const FhtGeometry& g, const FhtFusedTables& t, const FhtRgcArgs& a) {
@@ -152,7 +154,7 @@ bool fht_pair_pays(const FhtGeometry& g, const FhtFusedTables& t, const FhtRgcAr
     const double fused_us = 10 + waves * ((a.F + G - 1) / G + (G > 1 && !emit ? 1.0 : 0.0) + 0.25) * 34.7 *
                             (6.2 * t.taps + 300) / 1875 * ((long)tiles * G <= sms ? 0.67 : 1.0) *
                                      (G > 1 && !emit ? 1.1 : 1.0);
-    return pair_us < fused_us;
+    return pair_us < (a.F == 1 ? 0.95 : 1.0) * fused_us;
 }
 
 cudaError_t fht_rgc_pair(const FhtGeometry& g, const FhtFusedTables& t, const FhtRgcArgs& a,
