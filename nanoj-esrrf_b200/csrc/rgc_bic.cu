@@ -4,7 +4,8 @@
 //
 // Per frame: 2-point gradient on the raw frame (liveSRRF.cl:187-214), Catmull-Rom 2x resampling
 // of the gradient (:217-233), RGC on the 2x gradient grid with bicubic intensity (:238-401).
-// Each output pixel is one thread that walks the frames of a launch with its cumulants in
+// Launches without drift at M 2 and 4 take the paired-tap kernel (bic_pair.cuh).  Here each
+// output pixel is one thread that walks the frames of a launch with its cumulants in
 // registers; the reference instead relaunches per frame and read-modify-writes global memory.
 #include <math.h>
 

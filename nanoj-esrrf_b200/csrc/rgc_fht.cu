@@ -2,7 +2,8 @@
 // path: LiveSRRF_CL.prepareBuffersFHTinterpolation loads liveSRRF_noInterpolation.cl,
 // LiveSRRF_CL.java:462-579).
 //
-// Two kernels compute the same map:
+// Launches without drift that are large enough take the paired-tap kernel (rgc_pair.cuh,
+// fht_pair_pays); the others one of two kernels that compute the same map here:
 //  * fht_rgc_plain_kernel: one thread per output pixel, the reference's per-tap arithmetic
 //    (liveSRRF_noInterpolation.cl:245-393) on a separately computed Roberts-cross gradient
 //    (:138-159); handles frames with drift.  Cumulants are kept in registers across the frames

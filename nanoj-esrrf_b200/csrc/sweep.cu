@@ -6,9 +6,9 @@
 // combination, and its rolling analysis (gui/LiveSRRF_optimised_.java:276-389) recomputes every
 // frame once per block that contains it.  Here one captured CUDA graph per device does the work:
 //   per magnification: Fourier-interpolate every frame once (interp.cu);
-//   per radius: one fused-RGC launch over all frames that writes CGLH / sum-of-weights per frame
+//   per radius: one RGC launch over all frames that writes CGLH / sum-of-weights per frame
 //     (the tap loop is shared by every sensitivity and every block);
-//   per (sensitivity group, block group): one memory-bound launch that raises CGLH to the
+//   per (sensitivity group, block group): one launch that raises CGLH to the
 //     sensitivity, weights it by the intensity and reduces AVG/VAR/TAC2/INT over each block, FP64
 //     accumulators in registers.
 // With drift (the sweep's vibration correction: one shift per frame of the stack,
@@ -17,7 +17,7 @@
 // getInterpolatedValue at its shifted position, sampled once per magnification.
 // The bicubic sweep (the reference sweep with "Use FHT interpolation" off) computes the 2-point
 // gradients, their 2x resampling and the unit-gradient field of every frame once (none depends on
-// the magnification or radius); per (magnification, radius) the tabulated bicubic RGC writes
+// the magnification or radius); per (magnification, radius) the paired-tap or the tabulated RGC writes
 // CGLH / sum of weights and the bicubic intensity of every frame; the cumulant launches apply the
 // path's double (n - 1) division of TAC2, and every output gets the MP correction.
 //
