@@ -249,25 +249,38 @@ esrrf_status esrrf_handle::init_bic3d() {
         if (tbic_built) {
             CK(cudaMalloc(&d_u2, sizeof(float2) * bic_field_float2s(tbic, F)));
             CK(cudaMemsetAsync(d_u2, 0, sizeof(float2) * bic_field_float2s(tbic, F), stream));  // zero halo
-            CK(bic_pair_tables(bgeo, M, tpair));
-            const size_t px = (size_t)F * WM * HM;
-            if (!bic_pair_fits(tpair, ws, hs, M) || p.kernel != 0 ||
-                cudaMalloc(&d_nodes, sizeof(float2) * F * 4 * plane) != cudaSuccess ||
-                cudaMalloc(&d_own, sizeof(float) * px) != cudaSuccess ||
-                cudaMalloc(&d_edge, sizeof(float) * px) != cudaSuccess) {
-                // no such tables, or no room for its planes: the tabulated kernel takes every launch
-                cudaGetLastError();
-                bic_pair_tables_free(tpair);
-                cudaFree(d_nodes);
-                cudaFree(d_own);
-                cudaFree(d_edge);
-                d_nodes = nullptr;
-                d_own = d_edge = nullptr;
-            }
         }
     }
     CK(cudaMalloc(&d_mpmap, sizeof(float) * 3 * M * M * M));
-    return alloc_common(sizeof(float) * (size_t)W * H, (long)WM * HM * PM);
+    const esrrf_status r = alloc_common(sizeof(float) * (size_t)W * H, (long)WM * HM * PM);
+    if (r == ESRRF_OK && tbic_built && p.kernel == 0) take_pair_planes();
+    return r;
+}
+
+// The paired-tap form's buffers.  Without them the tabulated kernel takes every launch, so they come after
+// everything the handle cannot do without, and only where they leave room for what it allocates later (the
+// second output of a queued read-back) and 256 MB for the caller.
+void esrrf_handle::take_pair_planes() {
+    const size_t plane = (size_t)ws * hs, px = (size_t)F * WM * HM;
+    const size_t want = sizeof(float2) * F * 4 * plane + sizeof(float) * 2 * px;
+    const size_t later = sizeof(float) * 4 * (size_t)st.pixels + (size_t(256) << 20);
+    size_t avail = 0, all = 0;
+    if (bic_pair_tables(bgeo, p.magnification, tpair) != cudaSuccess ||
+        !bic_pair_fits(tpair, ws, hs, p.magnification) || cudaMemGetInfo(&avail, &all) != cudaSuccess ||
+        avail < want + later || cudaMalloc(&d_nodes, sizeof(float2) * F * 4 * plane) != cudaSuccess ||
+        cudaMalloc(&d_own, sizeof(float) * px) != cudaSuccess || cudaMalloc(&d_edge, sizeof(float) * px) != cudaSuccess) {
+        cudaGetLastError();
+        drop_pair_planes();
+    }
+}
+
+void esrrf_handle::drop_pair_planes() {
+    bic_pair_tables_free(tpair);
+    cudaFree(d_nodes);
+    cudaFree(d_own);
+    cudaFree(d_edge);
+    d_nodes = nullptr;
+    d_own = d_edge = nullptr;
 }
 
 esrrf_status esrrf_handle::init_fht() {
@@ -338,10 +351,7 @@ void esrrf_handle::release() {
     cudaFree(d_u3);
     bic_tables_free(tbic);
     cudaFree(d_u2);
-    bic_pair_tables_free(tpair);
-    cudaFree(d_nodes);
-    cudaFree(d_own);
-    cudaFree(d_edge);
+    drop_pair_planes();
     for (float* b : {d_fraw, d_planes, d_gz, d_gxi, d_gyi, d_gzi, d_mpmap, mfm.coeff, mfm.cos_t,
                      mfm.sin_t, mfm.shx, mfm.shy})
         cudaFree(b);
@@ -701,7 +711,14 @@ esrrf_status esrrf_handle::read_async(float* out) {
     CK(cudaSetDevice(device));
     if (frame_in_block == 0) return fail(ESRRF_ERR_STATE, "no frames accumulated in this block");
     const size_t bytes = sizeof(float) * 4 * (size_t)st.pixels;
-    if (!d_out2) CK(cudaMalloc(&d_out2, bytes));
+    if (!d_out2 && cudaMalloc(&d_out2, bytes) != cudaSuccess) {
+        // no room: give back the planes that a launch can do without
+        cudaGetLastError();
+        d_out2 = nullptr;
+        CK(cudaStreamSynchronize(stream));
+        drop_pair_planes();
+        CK(cudaMalloc(&d_out2, bytes));
+    }
     const int s = read_slot;
     read_slot ^= 1;
     float* dst = s ? d_out2 : d_out;
@@ -906,8 +923,9 @@ esrrf_status esrrf_read_gradients(esrrf_handle* h, float* out, size_t out_len) {
         // 2x-resampled gradient components of the first frame of the last push
         const size_t plane = (size_t)4 * h->ws * h->hs * h->P;
         // the paired form leaves no gradient planes: those of the first frame, from its float copy
+        // (the staging buffer is idle: a push has returned, and this call waits for its kernels)
         if (h->grad_stale &&
-            bic_prepare(h->d_fraw, 0, h->ws, h->hs, 1, (float*)h->d_nodes, h->d_gx, h->d_gy, h->d_gxi, h->d_gyi, h->stream) !=
+            bic_prepare(h->d_fraw, 0, h->ws, h->hs, 1, (float*)h->d_raw[0], h->d_gx, h->d_gy, h->d_gxi, h->d_gyi, h->stream) !=
                 cudaSuccess) {
             cudaGetLastError();
             return h->fail(ESRRF_ERR_CUDA, "gradient read-back failed");

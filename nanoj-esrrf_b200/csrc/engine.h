@@ -116,6 +116,8 @@ struct esrrf_handle {
     esrrf_status init_fht();
     esrrf_status init_bic3d();
     esrrf_status alloc_common(size_t raw_frame_bytes, long out_pixels);
+    void take_pair_planes();  // bicubic: the optional buffers of the paired-tap form
+    void drop_pair_planes();
     void release();
     esrrf_status reset_block();
     esrrf_status set_drift(const float* dx, const float* dy);
