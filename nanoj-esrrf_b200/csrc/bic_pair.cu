@@ -310,9 +310,12 @@ cudaError_t launch_cumulants(const BicCumArgs& c, cudaStream_t stream) {
 
 }  // namespace
 
-cudaError_t bic_pair_tables(const BicGeometry& g, int M, BicPairTables& t) {
-    t = BicPairTables();
-    if (M != 2 && M != 4) return cudaSuccess;
+namespace {
+
+// The table's (I + 1) x kNJ entries too, if `tab` is given.
+BicPairTables reach(const BicGeometry& g, int M, std::vector<float2>* tab) {
+    BicPairTables t;
+    if (M != 2 && M != 4) return t;
     // distances of i - 1/2 and j - 1/2 output pixels inside the disc of tSO raw pixels; d, the weight
     // and the cut-off in raw pixels, the reference's floats
     auto weight = [&](int i, int j, float& w, float& wd) {
@@ -327,16 +330,27 @@ cudaError_t bic_pair_tables(const BicGeometry& g, int M, BicPairTables& t) {
     float w, wd;
     int I = 0;
     while (I <= kMaxJ && weight(I + 1, 1, w, wd)) ++I;
-    if (I < 1 || I > kMaxJ) return cudaSuccess;
-    std::vector<float2> tab((size_t)(I + 1) * kNJ, make_float2(0.f, 0.f));
+    if (I < 1 || I > kMaxJ) return t;
+    if (tab) tab->assign((size_t)(I + 1) * kNJ, make_float2(0.f, 0.f));
     for (int i = 1; i <= I; ++i)
         for (int j = 1; j < kNJ && weight(i, j, w, wd); ++j) {
-            tab[(size_t)i * kNJ + j] = make_float2(w, wd);
+            if (tab) (*tab)[(size_t)i * kNJ + j] = make_float2(w, wd);
             t.J[i] = (signed char)j;
             t.taps += 4;  // a quadrant's distance stands for four taps
         }
     t.I = I;
     t.taps = t.taps * 4 / (M * M);  // nodes in an output's disc
+    return t;
+}
+
+}  // namespace
+
+BicPairTables bic_pair_reach(const BicGeometry& g, int M) { return reach(g, M, nullptr); }
+
+cudaError_t bic_pair_tables(const BicGeometry& g, int M, BicPairTables& t) {
+    std::vector<float2> tab;
+    t = reach(g, M, &tab);
+    if (t.I < 1) return cudaSuccess;
     cudaError_t e = cudaMalloc(&t.wt, sizeof(float2) * tab.size());
     if (e != cudaSuccess) return e;
     return cudaMemcpy(t.wt, tab.data(), sizeof(float2) * tab.size(), cudaMemcpyHostToDevice);
@@ -381,7 +395,7 @@ int pair_warps(const BicPairArgs& p, int M) {
 }  // namespace
 
 bool bic_pair_fits(const BicPairTables& t, int w, int h, int M) {
-    if (!t.wt || (long)h * M > 65535 || 2L * h > 65535 * 8L) return false;
+    if (t.I < 1 || (long)h * M > 65535 || 2L * h > 65535 * 8L) return false;
     return pair_warps(pair_args(t, w, h, M), M) >= 4;
 }
 
@@ -400,7 +414,7 @@ PairShape shape_of(const BicPairArgs& p, int M, int F, int sms) {
 // 512 x 512 at M4 2.1 ms against 5.4, 20 frames of 120 x 100 at M4 141 us / 229, 12 of 90 x 80 at M2 (radius
 // 3) 85 / 102, 12 of 37 x 29 at M4 87 / 63, 12 of 60 x 50 at M4 (radius 3) 188 / 128.
 bool bic_pair_pays(const BicPairTables& t, int w, int h, int M, int F) {
-    if (!t.wt || F > 65535 || (2L * w + 31) / 32 * F > (1 << 26)) return false;
+    if (t.I < 1 || F > 65535 || (2L * w + 31) / 32 * F > (1 << 26)) return false;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
     const int sms = sm_count(dev);
@@ -415,6 +429,25 @@ bool bic_pair_pays(const BicPairTables& t, int w, int h, int M, int F) {
                                    (0.35 + 0.65 * std::min(1.0, (double)ctas / slots)) +
                           1.25e-4 * w * h * F;
     return pair_us < tab_us;
+}
+
+bool bic_pair_pays_up_to(const BicPairTables& t, int w, int h, int M, int F) {
+    for (int f = F; f >= 1; --f)
+        if (bic_pair_pays(t, w, h, M, f)) return true;
+    return false;
+}
+
+// A frame of the tabulated form holds 19 input planes on the device (the frame and its gradients, the 2x
+// gradients and the padded unit-gradient field): launches within 2 GB of them.  The paired form adds its
+// two output planes (its nodes share the 2x gradients' memory), 2 M^2 input planes; its launches of few frames run
+// shorter segments, so they have the 4 GB of the Fourier path: 100 frames of 1024 x 1024 at M4 36.0
+// ms in launches of 9 (2 GB), 33.1 of 17 (4 GB), 32.7 of 25 (5.4 GB).
+int bic_launch_cap(const BicGeometry& g, int w, int h, int M, bool plain, int want) {
+    const double plane = sizeof(float) * (double)w * h;
+    const int f = (int)std::max(1.0, std::min((double)want, 2e9 / (19 * plane)));
+    const BicPairTables t = plain ? BicPairTables() : bic_pair_reach(g, M);
+    if (!bic_pair_fits(t, w, h, M) || !bic_pair_pays_up_to(t, w, h, M, f)) return f;
+    return (int)std::max(1.0, std::min((double)want, 4e9 / ((19 + 2.0 * M * M) * plane)));
 }
 
 cudaError_t bic_rgc_pair(const BicPairRun& r, const BicPairTables& t, cudaStream_t stream) {

@@ -139,11 +139,10 @@ esrrf_status esrrf_handle::init(const esrrf_params& params) {
         const int launches = (nb + fmax - 1) / fmax;
         F = (nb + launches - 1) / launches;
     } else if (p.frames_per_launch == 0 && mode == Mode::kBIC) {
-        // 2-D bicubic path: likewise at most 32 frames (100-frame blocks of 512 x 512 at M4: 4 %
-        // faster than 8), within ~2 GB of per-frame buffers (raw frame and its gradients, the 2x
-        // gradients and the padded unit-gradient field: ~19 input planes)
-        const double per_frame = 19.0 * sizeof(float) * (double)p.width * p.height;
-        const int fmax = (int)std::max(1.0, std::min(32.0, 2e9 / per_frame));
+        // 2-D bicubic path: likewise at most 32 frames (100-frame blocks of 512 x 512 at M4: 10 %
+        // faster than 9) within bic_launch_cap's memory
+        const int fmax = bic_launch_cap(bic_geometry(p.fwhm, p.sensitivity), p.width, p.height, p.magnification,
+                                        p.kernel != 0, 32);
         const int nb = std::max(1, p.n_frame_for_srrf);
         const int launches = (nb + fmax - 1) / fmax;
         F = (nb + launches - 1) / launches;
@@ -235,8 +234,14 @@ esrrf_status esrrf_handle::init_bic3d() {
     CK(cudaMalloc(&d_fraw, sizeof(float) * F * P * plane));
     CK(cudaMalloc(&d_gx, sizeof(float) * F * P * plane));
     CK(cudaMalloc(&d_gy, sizeof(float) * F * P * plane));
-    CK(cudaMalloc(&d_gxi, sizeof(float) * F * P * 4 * plane));
-    CK(cudaMalloc(&d_gyi, sizeof(float) * F * P * 4 * plane));
+    if (mode == Mode::kBIC) {
+        // one buffer: the paired form's nodes take the place of both (a launch runs one form)
+        CK(cudaMalloc(&d_gxi, sizeof(float) * 2 * F * 4 * plane));
+        d_gyi = d_gxi + F * 4 * plane;
+    } else {
+        CK(cudaMalloc(&d_gxi, sizeof(float) * F * P * 4 * plane));
+        CK(cudaMalloc(&d_gyi, sizeof(float) * F * P * 4 * plane));
+    }
     if (mode == Mode::k3D) {
         CK(cudaMalloc(&d_planes, sizeof(float) * F * P * plane));
         CK(cudaMalloc(&d_gz, sizeof(float) * F * P * plane));
@@ -257,29 +262,29 @@ esrrf_status esrrf_handle::init_bic3d() {
     return r;
 }
 
-// The paired-tap form's buffers.  Without them the tabulated kernel takes every launch, so they come after
-// everything the handle cannot do without, and only where they leave room for what it allocates later (the
-// second output of a queued read-back) and 256 MB for the caller.
+// The paired-tap form's two planes, where launches of this handle take it.  Without them the tabulated
+// kernel takes every launch, so they come after everything the handle cannot do without, and only where
+// they leave room for what it allocates later (the second output of a queued read-back) and 256 MB for
+// the caller.
 void esrrf_handle::take_pair_planes() {
-    const size_t plane = (size_t)ws * hs, px = (size_t)F * WM * HM;
-    const size_t want = sizeof(float2) * F * 4 * plane + sizeof(float) * 2 * px;
+    const int M = p.magnification;
+    const BicPairTables t = bic_pair_reach(bgeo, M);
+    if (!bic_pair_fits(t, ws, hs, M) || !bic_pair_pays_up_to(t, ws, hs, M, F)) return;
+    const size_t px = (size_t)F * WM * HM, want = sizeof(float) * 2 * px;
     const size_t later = sizeof(float) * 4 * (size_t)st.pixels + (size_t(256) << 20);
     size_t avail = 0, all = 0;
-    if (bic_pair_tables(bgeo, p.magnification, tpair) != cudaSuccess ||
-        !bic_pair_fits(tpair, ws, hs, p.magnification) || cudaMemGetInfo(&avail, &all) != cudaSuccess ||
-        avail < want + later || cudaMalloc(&d_nodes, sizeof(float2) * F * 4 * plane) != cudaSuccess ||
-        cudaMalloc(&d_own, sizeof(float) * px) != cudaSuccess || cudaMalloc(&d_edge, sizeof(float) * px) != cudaSuccess) {
+    if (cudaMemGetInfo(&avail, &all) != cudaSuccess || avail < want + later ||
+        cudaMalloc(&d_own, want) != cudaSuccess || bic_pair_tables(bgeo, M, tpair) != cudaSuccess) {
         cudaGetLastError();
         drop_pair_planes();
+        return;
     }
+    d_edge = d_own + px;
 }
 
 void esrrf_handle::drop_pair_planes() {
     bic_pair_tables_free(tpair);
-    cudaFree(d_nodes);
     cudaFree(d_own);
-    cudaFree(d_edge);
-    d_nodes = nullptr;
     d_own = d_edge = nullptr;
 }
 
@@ -352,6 +357,7 @@ void esrrf_handle::release() {
     bic_tables_free(tbic);
     cudaFree(d_u2);
     drop_pair_planes();
+    if (mode == Mode::kBIC) d_gyi = nullptr;  // part of d_gxi
     for (float* b : {d_fraw, d_planes, d_gz, d_gxi, d_gyi, d_gzi, d_mpmap, mfm.coeff, mfm.cos_t,
                      mfm.sin_t, mfm.shx, mfm.shy})
         cudaFree(b);
@@ -511,7 +517,7 @@ esrrf_status esrrf_handle::process_chunk_bic3d(const void* src, bool is_u16, int
     const bool paired = mode == Mode::kBIC && no_drift && bic_pair_pays(tpair, ws, hs, p.magnification, F_now);
     grad_stale = paired;
     if (paired) {
-        CK(bic_nodes(src, is_u16 ? 1 : 0, ws, hs, F_now, d_fraw, d_nodes, stream));
+        CK(bic_nodes(src, is_u16 ? 1 : 0, ws, hs, F_now, d_fraw, (float2*)d_gxi, stream));
         launches += 1;
     } else if (mode == Mode::kBIC) {
         CK(bic_prepare(src, is_u16 ? 1 : 0, W, H, F_now, d_fraw, d_gx, d_gy, d_gxi, d_gyi, stream));
@@ -524,7 +530,7 @@ esrrf_status esrrf_handle::process_chunk_bic3d(const void* src, bool is_u16, int
     if (timing) CK(cudaEventRecord(e1, stream));
     if (paired) {
         BicPairRun r{};
-        r.U = d_nodes;
+        r.U = (const float2*)d_gxi;
         r.fraw = d_fraw;
         r.wsum = tbic.wsum;
         r.own = d_own;

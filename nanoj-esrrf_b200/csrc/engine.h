@@ -55,7 +55,8 @@ struct esrrf_handle {
     float* d_fraw = nullptr;    // [F][P][hs][ws] float frames / aligned planes
     float* d_planes = nullptr;  // [F][P][hs][ws] split planes before alignment (3-D)
     float* d_gz = nullptr;
-    float* d_gxi = nullptr;     // [F][P][2hs][2ws]
+    float* d_gxi = nullptr;     // [F][P][2hs][2ws]; 2-D bicubic: d_gyi behind it, or the paired form's unit
+                                // gradient at the nodes, float2 [F][2hs][2ws], in the place of both
     float* d_gyi = nullptr;
     float* d_gzi = nullptr;
     float* d_mpmap = nullptr;   // [3][M^2 or M^3]
@@ -65,8 +66,7 @@ struct esrrf_handle {
     bool tbic_built = false;
     float2* d_u2 = nullptr;     // [F][2hs][2ws] padded unit gradient field (2-D bicubic)
     esrrf::BicPairTables tpair; // paired-tap form of the bicubic RGC (null where it does not apply)
-    float2* d_nodes = nullptr;  // [F][2hs][2ws] unit gradient at the nodes, for it
-    float* d_own = nullptr;     // [F][HM][WM] its two planes
+    float* d_own = nullptr;     // [2][F][HM][WM] its two planes, d_edge the second
     float* d_edge = nullptr;
     bool grad_stale = false;    // bicubic: the last push took the paired form, which leaves no gradient planes
 

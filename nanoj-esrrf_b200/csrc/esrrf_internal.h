@@ -290,11 +290,15 @@ struct BicPairTables {
     int taps = 0;          // taps of an output pixel
     signed char J[16] = {};
 };
-cudaError_t bic_pair_tables(const BicGeometry& g, int M, BicPairTables& t);  // t.wt null: not supported
+BicPairTables bic_pair_reach(const BicGeometry& g, int M);  // all but wt; I 0: not supported
+cudaError_t bic_pair_tables(const BicGeometry& g, int M, BicPairTables& t);
 void bic_pair_tables_free(BicPairTables& t);
 bool bic_pair_fits(const BicPairTables& t, int w, int h, int M);
-// Whether it is the faster form for a launch of F frames.
+// Whether it is the faster form for a launch of F frames; for one of 1 .. F frames.
 bool bic_pair_pays(const BicPairTables& t, int w, int h, int M, int F);
+bool bic_pair_pays_up_to(const BicPairTables& t, int w, int h, int M, int F);
+// The most frames a launch of the 2-D bicubic engine may have within its memory budget, of `want` at most.
+int bic_launch_cap(const BicGeometry& g, int w, int h, int M, bool plain, int want);
 // raw -> float frames and the unit gradient at the nodes [F][2h][2w]
 cudaError_t bic_nodes(const void* raw, int is_u16, int w, int h, int F, float* fraw, float2* U, cudaStream_t stream);
 struct BicPairRun {

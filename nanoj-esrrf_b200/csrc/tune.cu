@@ -121,10 +121,10 @@ std::vector<int> candidates(const esrrf_params& p, int n) {
         per_frame = 5.0 * sizeof(float) * (double)p.width * p.magnification * p.height * p.magnification;
     } else {
         targets = {8, 16, 25, 32, 50, 64};
-        per_frame = 19.0 * sizeof(float) * (double)p.width * p.height;
-        budget = 2e9;
     }
-    const int fcap = (int)std::max(1.0, std::floor(budget / per_frame));
+    const int fcap = per_frame > 0 ? (int)std::max(1.0, std::floor(budget / per_frame))
+                                   : bic_launch_cap(bic_geometry(p.fwhm, p.sensitivity), p.width, p.height,
+                                                    p.magnification, p.kernel != 0, targets.back());
     std::vector<int> out;
     for (int f : targets) {
         f = std::min({f, fcap, n});
@@ -214,14 +214,14 @@ esrrf_status tune_engine(const esrrf_params& params, TuneChoice& out, std::strin
     }
     // one block of synthetic frames (at most 200: the per-launch costs show within that)
     const int n = std::min(p.n_frame_for_srrf, 200);
-    const std::vector<int> Fs = candidates(p, n);
-    std::vector<int> forms = {kRgc3dAuto};
-    if (p.n_planes > 0 && p.kernel == 0) forms = {kRgc3dTwoCells, kRgc3dSlab, kRgc3dL1};
     if (cudaSetDevice(dev) != cudaSuccess) {
         cudaGetLastError();
         msg = "autotuner: cudaSetDevice failed";
         return ESRRF_ERR_CUDA;
     }
+    const std::vector<int> Fs = candidates(p, n);
+    std::vector<int> forms = {kRgc3dAuto};
+    if (p.n_planes > 0 && p.kernel == 0) forms = {kRgc3dTwoCells, kRgc3dSlab, kRgc3dL1};
     float* d_frames = nullptr;
     float* d_out = nullptr;
     const long planes_out = p.n_planes > 0 ? (long)p.n_planes * p.magnification : 1;

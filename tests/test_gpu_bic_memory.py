@@ -105,3 +105,27 @@ def test_planes_are_given_back_for_a_queued_read(esrrf_mod):
         eng.release()
     for k in range(4):
         assert rel_err(out[0][k], want[k]) < TOL, k
+
+
+def test_launch_size_counts_the_paired_forms_planes(esrrf_mod, tmp_path, monkeypatch):
+    """A launch's frames are limited by the memory that they hold in the form they take: 19 input planes and the
+    paired form's 2 M^2, 4 GB in all.  What the handle holds besides is counted from its arrays: accumulators
+    (4 x 8 bytes an output pixel), previous values, output and sums of weights (6 floats), and the staging."""
+    import torch
+    torch.zeros(1, device="cuda")
+    engine(esrrf_mod, 64, 64, 4, 25).release()
+    for w, h, M in ((1024, 1024, 4), (1300, 900, 2)):
+        before = free_bytes()
+        eng = engine(esrrf_mod, w, h, M, 100)
+        held, F = before - free_bytes(), eng.framesPerLaunch()
+        eng.release()
+        rest = (4 * 8 + 6 * 4) * w * h * M * M + 2 * F * 4 * w * h
+        assert held <= 4e9 + rest + 64 * MB, (held, F)
+        assert F >= 17  # and still long enough launches
+    monkeypatch.setenv("ESRRF_TUNE_CACHE", str(tmp_path / "tune.txt"))
+    eng = engine(esrrf_mod, 1024, 1024, 4, 100, framesPerLaunch=-1)
+    try:
+        tried = [c["frames_per_launch"] for c in eng.tuneReport()["candidates"]]
+    finally:
+        eng.release()
+    assert max(tried) * (19 + 2 * 16) * 4 * 1024 * 1024 <= 4e9, tried
