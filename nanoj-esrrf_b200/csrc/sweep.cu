@@ -240,11 +240,10 @@ struct Shard {
     float* d_fraw = nullptr;
     float* d_gx = nullptr;
     float* d_gy = nullptr;
-    float* d_gxi = nullptr;
+    float* d_gxi = nullptr;     // d_gyi behind it; then the unit gradient at the nodes, if an entry is paired
     float* d_gyi = nullptr;
     float2* d_u2 = nullptr;
-    float2* d_nodes = nullptr;  // unit gradient at the nodes (entries with a paired-tap form)
-    bool tabulated = false;     // some entry runs the tabulated kernel
+    bool tabulated = true;      // some entry runs the tabulated kernel
     float* d_mpmap = nullptr;
     std::vector<size_t> offsets;  // local layout: per (mp entry, radius entry) in order
     size_t total = 0;
@@ -279,6 +278,11 @@ struct Shard {
     esrrf_status tc_check();
     esrrf_status run_device(const void* d_frames, int is_u16, float* d_out, float* h_out = nullptr);
     void release();
+    // bytes that a host run allocates (its first one)
+    size_t staging_bytes() const { return sizeof(float) * (total + (size_t)T * w * h); }
+    cudaError_t stage(void** p, size_t bytes);
+    void take_planes(size_t reserve);
+    void drop_planes();
 };
 
 #define SK(call, what)                                         \
@@ -394,8 +398,8 @@ esrrf_status Shard::enqueue_bic(const void* frames, int is_u16, float* out, floa
         SK(unit_grad2d(d_gxi, d_gyi, w, h, T, mp[0].btab[0], d_u2, stream), "unit gradient");
         ++launches;
     }
-    if (d_nodes) {
-        SK(bic_nodes(frames, is_u16, w, h, T, d_fraw, d_nodes, stream), "gradients");
+    if (d_edge) {  // after unit_grad2d: the nodes overwrite the 2x gradients
+        SK(bic_nodes(frames, is_u16, w, h, T, d_fraw, (float2*)d_gxi, stream), "gradients");
         ++launches;
     }
     size_t oi = 0;
@@ -405,7 +409,7 @@ esrrf_status Shard::enqueue_bic(const void* frames, int is_u16, float* out, floa
         for (size_t e = 0; e < m.ri.size(); ++e, ++oi) {
             if (m.bpair[e].wt) {
                 BicPairRun r{};
-                r.U = d_nodes;
+                r.U = (const float2*)d_gxi;
                 r.fraw = d_fraw;
                 r.wsum = m.btab[e].wsum;
                 r.edge = d_edge;
@@ -488,10 +492,8 @@ void Shard::release() {
         cudaFree(m.d_shift);
     }
     fht_drift_tables_free(dtab);
-    for (float* b : {d_fraw, d_gx, d_gy, d_gxi, d_gyi, d_mpmap}) cudaFree(b);
+    for (float* b : {d_fraw, d_gx, d_gy, d_gxi, d_mpmap}) cudaFree(b);
     cudaFree(d_u2);
-    cudaFree(d_nodes);
-    d_nodes = nullptr;
     d_fraw = d_gx = d_gy = d_gxi = d_gyi = d_mpmap = nullptr;
     d_u2 = nullptr;
     mp.clear();
@@ -547,6 +549,7 @@ esrrf_status Shard::create_bic(const std::vector<float>& radii) {
             pady = std::max(pady, t.pady);
             m.bgeo.push_back(g);
             m.btab.push_back(t);
+            m.bpair.push_back(BicPairTables());
             offsets.push_back(total);
             total += (size_t)sens.size() * bstart.size() * 4 * P;
         }
@@ -565,42 +568,15 @@ esrrf_status Shard::create_bic(const std::vector<float>& radii) {
     if ((e = cudaMalloc(&d_fraw, sizeof(float) * T * plane)) != cudaSuccess ||
         (e = cudaMalloc(&d_gx, sizeof(float) * T * plane)) != cudaSuccess ||
         (e = cudaMalloc(&d_gy, sizeof(float) * T * plane)) != cudaSuccess ||
-        (e = cudaMalloc(&d_gxi, sizeof(float) * T * 4 * plane)) != cudaSuccess ||
-        (e = cudaMalloc(&d_gyi, sizeof(float) * T * 4 * plane)) != cudaSuccess ||
+        (e = cudaMalloc(&d_gxi, sizeof(float) * 2 * T * 4 * plane)) != cudaSuccess ||
         (e = cudaMalloc(&d_u2, sizeof(float2) * field)) != cudaSuccess ||
         (e = cudaMalloc(&d_mpmap, sizeof(float) * 3 * maxM * maxM)) != cudaSuccess ||
         (e = cudaMalloc(&d_interp, sizeof(float) * (size_t)T * maxP)) != cudaSuccess ||
         (e = cudaMalloc(&d_cg, sizeof(float) * (size_t)T * maxP)) != cudaSuccess)
         return fail_cuda(e, "sweep buffers");
+    d_gyi = d_gxi + T * 4 * plane;
     if ((e = cudaMemsetAsync(d_u2, 0, sizeof(float2) * field, stream)) != cudaSuccess)  // zero halo
         return fail_cuda(e, "sweep buffers");
-    // paired-tap forms where they are the faster ones and their planes leave room for the staging of a
-    // host run
-    bool some = false;
-    for (auto& m : mp)
-        for (size_t i = 0; i < m.ri.size(); ++i) {
-            BicPairTables t;
-            if ((e = bic_pair_tables(m.bgeo[i], m.M, t)) != cudaSuccess) return fail_cuda(e, "RGC tables");
-            if (!bic_pair_fits(t, w, h, m.M) || !bic_pair_pays(t, w, h, m.M, T)) bic_pair_tables_free(t);
-            some = some || t.wt;
-            m.bpair.push_back(t);
-        }
-    if (some) {
-        const size_t edge = sizeof(float) * (size_t)T * maxP, nodes = sizeof(float2) * (size_t)T * 4 * plane;
-        const size_t later = sizeof(float) * (total + (size_t)T * plane) + (size_t(256) << 20);
-        size_t avail = 0, all = 0;
-        if (cudaMemGetInfo(&avail, &all) != cudaSuccess || avail < edge + nodes + later ||
-            cudaMalloc(&d_edge, edge) != cudaSuccess || cudaMalloc(&d_nodes, nodes) != cudaSuccess) {
-            cudaGetLastError();
-            cudaFree(d_edge);
-            d_edge = nullptr;
-            d_nodes = nullptr;
-            for (auto& m : mp)
-                for (auto& t : m.bpair) bic_pair_tables_free(t);
-        }
-    }
-    for (auto& m : mp)
-        for (auto& t : m.bpair) tabulated = tabulated || !t.wt;
     if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return fail_cuda(e, "sync");
     return ESRRF_OK;
 }
@@ -665,21 +641,79 @@ esrrf_status Shard::create(const std::vector<float>& radii, int interp) {
         (e = cudaMalloc(&d_interp, sizeof(float) * (size_t)T * maxP)) != cudaSuccess ||
         (e = cudaMalloc(&d_cg, sizeof(float) * (size_t)T * maxP)) != cudaSuccess)
         return fail_cuda(e, "sweep buffers");
-    if (!drift) {
-        // the paired-tap kernel's second plane, where it leaves room for the staging of a host run;
-        // without it the fused kernel runs
-        const size_t want = sizeof(float) * (size_t)T * maxP;
-        const size_t later = sizeof(float) * (total + (size_t)T * w * h) + (size_t(256) << 20);
-        size_t avail = 0, all = 0;
-        if (cudaMemGetInfo(&avail, &all) != cudaSuccess || avail < want + later ||
-            cudaMalloc(&d_edge, want) != cudaSuccess) {
-            cudaGetLastError();
-            d_edge = nullptr;
-        }
-    }
     if (drift && (e = fht_drift_tables_alloc(maxS, T, maxP, dtab)) != cudaSuccess) return fail_cuda(e, "drift tables");
     if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return fail_cuda(e, "sync");
     return ESRRF_OK;
+}
+
+// The paired-tap kernels' second plane, if an entry would take them and `reserve` bytes stay free besides;
+// without it the fused or the tabulated kernel runs.  Called for one shard after another, once every shard
+// has what it cannot do without (two shards may be on one device).
+void Shard::take_planes(size_t reserve) {
+    if (drift || cudaSetDevice(device) != cudaSuccess) return;
+    long maxP = 0;
+    bool some = false;
+    for (auto& m : mp) {
+        const long P = (long)w * m.M * h * m.M;
+        maxP = std::max(maxP, P);
+        for (size_t i = 0; i < m.ri.size() && !some; ++i) {
+            if (bic) {
+                const BicPairTables t = bic_pair_reach(m.bgeo[i], m.M);
+                some = bic_pair_fits(t, w, h, m.M) && bic_pair_pays(t, w, h, m.M, T);
+            } else {
+                FhtRgcArgs a{};
+                a.W = m.plan.WM;
+                a.H = m.plan.HM;
+                a.F = T;
+                a.cg_out = a.edge = d_cg;  // whether they are there is what counts
+                some = fht_pair_pays(m.geo[i], m.tables[i], a);
+            }
+        }
+    }
+    const size_t want = sizeof(float) * (size_t)T * maxP;
+    size_t avail = 0, all = 0;
+    if (!some || cudaMemGetInfo(&avail, &all) != cudaSuccess || avail < want + reserve ||
+        cudaMalloc(&d_edge, want) != cudaSuccess) {
+        cudaGetLastError();
+        d_edge = nullptr;
+        return;
+    }
+    if (!bic) return;
+    tabulated = false;
+    for (auto& m : mp)
+        for (size_t i = 0; i < m.ri.size(); ++i) {
+            BicPairTables& t = m.bpair[i];
+            const BicPairTables r = bic_pair_reach(m.bgeo[i], m.M);
+            if (!bic_pair_fits(r, w, h, m.M) || !bic_pair_pays(r, w, h, m.M, T)) {
+                tabulated = true;
+            } else if (bic_pair_tables(m.bgeo[i], m.M, t) != cudaSuccess) {
+                cudaGetLastError();
+                drop_planes();
+                return;
+            }
+        }
+}
+
+void Shard::drop_planes() {
+    if (stream) cudaStreamSynchronize(stream);
+    if (exec) cudaGraphExecDestroy(exec);  // it names the plane
+    if (graph) cudaGraphDestroy(graph);
+    exec = nullptr;
+    graph = nullptr;
+    for (auto& m : mp)
+        for (auto& t : m.bpair) bic_pair_tables_free(t);
+    tabulated = true;
+    cudaFree(d_edge);
+    d_edge = nullptr;
+}
+
+// A host run's buffer; the plane that a run can do without makes room for it.
+cudaError_t Shard::stage(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation || !d_edge) return e;
+    cudaGetLastError();
+    drop_planes();
+    return cudaMalloc(p, bytes);
 }
 
 // Reads every plan's tensor-core failure flag after the stream has drained.
@@ -1069,6 +1103,16 @@ esrrf_status esrrf_sweep_create(const esrrf_sweep_params* sp, esrrf_sweep** out)
     for (auto& t : th) t.join();
     for (size_t i = 0; i < s->shards.size(); ++i)
         if (rs[i] != ESRRF_OK) return bail(rs[i], s->shards[i]->err);
+    int current = 0;
+    cudaGetDevice(&current);
+    for (Shard* sh : s->shards) {
+        // room for the host runs of every shard on the device, and 256 MB for the caller
+        size_t reserve = size_t(256) << 20;
+        for (const Shard* o : s->shards)
+            if (o->device == sh->device) reserve += o->staging_bytes();
+        sh->take_planes(reserve);
+    }
+    cudaSetDevice(current);  // the caller's
     *out = s;
     return ESRRF_OK;
 }
@@ -1106,8 +1150,9 @@ esrrf_status esrrf_sweep_run(esrrf_sweep* s, const void* frames, int is_u16, flo
     auto work = [&](size_t i) -> esrrf_status {
         Shard* sh = s->shards[i];
         if (cudaSetDevice(sh->device) != cudaSuccess) return sh->fail(ESRRF_ERR_CUDA, "cudaSetDevice failed");
-        if (!sh->d_in) SKS(cudaMalloc(&sh->d_in, sizeof(float) * (size_t)s->p.width * s->p.height * sh->T), "input buffer");
-        if (!sh->d_outbuf) SKS(cudaMalloc(&sh->d_outbuf, sizeof(float) * sh->total), "output buffer");
+        if (!sh->d_in)
+            SKS(sh->stage(&sh->d_in, sizeof(float) * (size_t)s->p.width * s->p.height * sh->T), "input buffer");
+        if (!sh->d_outbuf) SKS(sh->stage((void**)&sh->d_outbuf, sizeof(float) * sh->total), "output buffer");
         SKS(cudaMemcpyAsync(sh->d_in, (const unsigned char*)frames + fbytes * sh->f0, fbytes * sh->T,
                             cudaMemcpyHostToDevice, sh->stream), "input copy");
         if (overlap) return sh->run_device(sh->d_in, is_u16, sh->d_outbuf, out);
