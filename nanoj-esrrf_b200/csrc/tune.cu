@@ -72,8 +72,10 @@ std::string cache_path() {
 std::string key_of(const esrrf_params& p, const std::string& devname) {
     std::ostringstream k;
     const bool fht = p.n_planes == 0 && p.interp == ESRRF_INTERP_FHT;
-    k << "v1|" << devname << "|" << (p.n_planes > 0 ? "3d" : fht ? "fht" : "bic") << "|" << p.width << "x"
-      << p.height << "|M" << p.magnification << "|";
+    // the version stands for the kernels that were timed, results of others are not reused: 2 in the 2-D
+    // paths since the paired-tap forms
+    k << (p.n_planes > 0 ? "v1|" : "v2|") << devname << "|" << (p.n_planes > 0 ? "3d" : fht ? "fht" : "bic") << "|"
+      << p.width << "x" << p.height << "|M" << p.magnification << "|";
     if (fht) k << "box" << fht_geometry(p.magnification, p.fwhm, 1).S;
     else k << "r" << p.fwhm;
     k << "|n" << p.n_frame_for_srrf << "|iw" << p.int_weighting << "|planes" << p.n_planes << "|k" << p.kernel;
