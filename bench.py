@@ -410,10 +410,13 @@ def run_reference(args, world, rank):
 
 TRAFFIC_SUMMARIES = {"rgc_fused_fht512": "rgc_pair_fht512.md", "rgc_fused_bic512": "bic_pair_bic512.md",
                      "rgc_fused_fht512_drift": "rgc_fused_drift_fht512.md"}
-# the kernel sources each summary's counts depend on
+# the RGC form each summary's counts are of
+SUMMARY_FORMS = {"rgc_fused_fht512": "fht_rgc_pair", "rgc_fused_bic512": "bic_pair",
+                 "rgc_fused_fht512_drift": "fht_rgc_fused"}
+# the sources each summary's counts depend on: the kernels, and the host code that lays a launch out
 SUMMARY_SOURCES = {
-    "rgc_fused_fht512": ["rgc_pair.cuh"],
-    "rgc_fused_bic512": ["bic_pair.cuh"],
+    "rgc_fused_fht512": ["rgc_pair.cuh", "rgc_pair.cu", "pair_shape.cu", "device_common.cuh"],
+    "rgc_fused_bic512": ["bic_pair.cuh", "bic_pair.cu", "pair_shape.cu", "device_common.cuh"],
     "rgc_fused_fht512_drift": ["fht_fused.cuh", "rgc_fht_drift.cu"],
 }
 
@@ -458,6 +461,35 @@ def summary_stale(kernel):
         return (f"profiles/{name} was captured from other kernel sources (sha {recorded}, now "
                 f"{source_sha(kernel)}): re-capture before quoting its figures")
     return None
+
+
+def rgc_form(bic, kernel, drift, counts, chunks, plain_count):
+    """The RGC form the engine's launches took, by their kernel counts: `counts`, each block's; `chunks`,
+    launches of a block; `plain_count`, kernels of one Fourier launch with the plain kernel.  A Fourier launch
+    has the interpolation's kernels and one fused, or a paired and its cumulants as the plain form its gradients
+    and RGC; a bicubic one three paired, five tabulated or four plain."""
+    if kernel == "plain":
+        return "bic_rgc" if bic else "fht_rgc_plain"
+    if drift:
+        return "bic_rgc" if bic else "fht_rgc_fused"
+    forms = ({3: "bic_pair", 5: "bic_tab", 4: "bic_rgc"} if bic else
+             {plain_count: "fht_rgc_pair", plain_count - 1: "fht_rgc_fused"})
+    got = {forms.get(c / chunks, "several forms") for c in counts}
+    return got.pop() if len(got) == 1 else "several forms"
+
+
+def plain_launch_count(width, height, M, fwhm, S, local):
+    """Kernels of a Fourier launch with the plain RGC."""
+    import esrrf
+
+    eng = esrrf.LiveSRRF_CL()
+    eng.initialise(width, height, M, fwhm, S, 1, 1, chosenDevice=local, kernel="plain")
+    try:
+        eng.resetFramePosition()
+        eng.calculateSRRF(np.zeros((1, height, width), np.uint16))
+        return eng.lastTiming()[2]
+    finally:
+        eng.release()
 
 
 def shard_blocks(world, rank, n_blocks, nf):
@@ -626,7 +658,7 @@ def run_ours(args, world, rank, local):
     frame_bytes = h * w * 2
     launches = [0]
     rgc_ms = [0.0]
-    rgc_n = [0]
+    block_launches = set()
 
     fp = ctypes.POINTER(ctypes.c_float)
 
@@ -644,6 +676,7 @@ def run_ours(args, world, rank, local):
                 H, ctypes.c_void_p(base + b * nf * frame_bytes), nf))
             _, r_ms, nl = eng.lastTiming()
             launches[0] += nl + 1
+            block_launches.add(nl)
             rgc_ms[0] += r_ms
             esrrf._lib.check(H, L.esrrf_read_srrf_device(H, ctypes.c_void_p(d_out[b].data_ptr())))
 
@@ -707,8 +740,11 @@ def run_ours(args, world, rank, local):
     value = world * mpxf / t_step
     e2e_value = world * mpxf / e2e_step
 
-    # roofline of the dominant kernel (fused RGC), per launch
-    launches_rgc = args.steps * n_blocks * ((nf + F - 1) // F)
+    # roofline of the RGC (its kernels between the engine's events), per launch
+    chunks = (nf + F - 1) // F
+    form = rgc_form(bic, args.kernel, args.drift, block_launches, chunks,
+                    0 if bic else plain_launch_count(w, h, M, fwhm, S, local))
+    launches_rgc = args.steps * n_blocks * chunks
     avg_launch_s = (rgc_total_ms / 1000.0) / max(1, launches_rgc)
     taps = bic_taps_per_pixel(M, fwhm) if bic else taps_per_pixel(M, fwhm)
     peaks, peak_src = load_peaks()
@@ -729,8 +765,10 @@ def run_ours(args, world, rank, local):
                      and args.frames is None and not args.block and not args.no_cpu_baseline) else None)
     summary_key = f"rgc_{args.kernel}_{args.workload}" + ("_drift" if args.drift else "")
     stale = summary_stale(summary_key)
+    if not stale and form != SUMMARY_FORMS[summary_key]:
+        stale = f"profiles/{TRAFFIC_SUMMARIES[summary_key]} is of {SUMMARY_FORMS[summary_key]}, the launches took {form}"
     traffic = None if stale else read_traffic_summary(summary_key)
-    # the kernel's real limit is instruction issue: warp instructions per launch (ncu count per
+    # the RGC's real limit is instruction issue: warp instructions per launch (ncu count per
     # frame x frames) over the live launch time, against one warp instruction per cycle per
     # scheduler (148 SMs x 4) at the sampled SM clock
     clocks = clk.summary()
@@ -741,11 +779,11 @@ def run_ours(args, world, rank, local):
     elif ipf and avg_launch_s > 0:
         mhz = clocks.get("sm_mhz") or 1965.0
         peak_issue = 148 * 4 * mhz * 1e6
-        got = ipf * (nf / ((nf + F - 1) // F)) / avg_launch_s  # mean frames per launch
+        got = ipf * (nf / chunks) / avg_launch_s  # mean frames per launch
         roofline_issue = {"achieved": got, "peak": peak_issue, "unit": "warp instructions/s",
                           "frac": got / peak_issue, "instructions_per_frame": ipf,
-                          "source": "instructions per frame from the committed ncu summary of this "
-                                    "kernel source (sha recorded there), launch time live"}
+                          "source": "instructions per frame of the timed kernels from the committed ncu "
+                                    "summary of this source (sha recorded there), launch time live"}
     line = {
         "metric": f"input Mpx*frames/s (eSRRF {path_label(args.workload)})",
         "value": value, "unit": "Mpx*frames/s", "n_gpus": world, "steps": args.steps,
@@ -754,7 +792,7 @@ def run_ours(args, world, rank, local):
         "config": {"workload": f"{args.workload}: {w}x{h}x{n} uint16, M{M}, radius {fwhm}, S{S}, "
                                f"{'bicubic interpolation, MP correction, ' if bic else ''}"
                                f"AVG+VAR+TAC2+INT, blocks of {nf}",
-                   "kernel": "bicubic" if bic else args.kernel,
+                   "kernel": form,
                    "frames_per_launch": F,
                    "l2": (f"inputs ({stack.nbytes / 1e6:.0f} MB) larger than L2" if stack.nbytes > 126e6 else
                           f"inputs ({stack.nbytes / 1e6:.1f} MB) fit in L2, not flushed between steps "
@@ -771,8 +809,7 @@ def run_ours(args, world, rank, local):
         "roofline": {"bound": "hbm", "achieved": achieved_gbs, "peak": peaks["hbm_gbs"],
                      "unit": "GB/s", "frac": achieved_gbs / peaks["hbm_gbs"],
                      "traffic": traffic, "peak_source": peak_src,
-                     "kernel": (("bic_pair" if args.kernel == "fused" else "bic_rgc") if bic else "fht_rgc_pair" if args.kernel == "fused" and not args.drift
-                                else f"fht_rgc_{args.kernel}"),
+                     "kernel": form,
                      "avg_launch_ms": avg_launch_s * 1e3,
                      "alg_bytes_per_launch": alg_bytes_launch},
         "roofline_fp32": {"achieved": achieved_tflops, "peak": FP32_PEAK_NOMINAL_TFLOPS,
