@@ -130,9 +130,10 @@ cudaError_t fht_pair_tables(const FhtGeometry& g, FhtFusedTables& t, cudaStream_
 // modelled, each in proportion to its instructions for the box's taps: 0.18 us per row and warp here
 // with segments up to 100 rows, 0.13 from 400 rows on (the widest boxes a fifth more), 34.7 us per tile
 // and frame for the fused kernel (0.67 of that where every SM has one tile at most; a tenth more
-// with several frame groups, which add into the sums with atomics).  On 56 launches from 48 x 48 to
-// 900 x 450 with boxes of 6 to 32 the rule takes the slower kernel only where they are within 5 %;
-// for one frame the fused kernel stays unless the other is ahead by as much (221 x 163 at M4, box 10:
+// with several frame groups, which add into the sums with atomics).  Of 521 launches that it gives to this
+// kernel, drawn from 4 x 4 to 700 x 700 pixels at M 1 to 13, boxes of 4 to 32 and 1 to 50 frames, four are
+// slower by 4 to 10 % (250 to 320 us of one or two frames), the others 0.57 of the fused kernel's time; for one
+// frame the fused kernel stays unless the other is ahead by as much (221 x 163 at M4, box 10:
 // modelled 49.0 / 49.7 us, measured 5 us behind).
 // Paired against fused, one block: 100 frames of 512 x 512 at M4 15.1 / 24.7 ms, 10 of 128 x 128 161 /
 // 229 us, one of 256 x 256 103 / 96 us, one of 128 x 128 82 / 39 us.

@@ -144,9 +144,13 @@ __device__ __forceinline__ void pair_far(int y, float* __restrict__ P, float* __
 
 // Column distance i = fi > 0 whose chord is the rows -J .. J: K sources x (2J + 1) pairs of taps.
 // P, M: the lane's output columns at X - i and X + i.  one: the opposite taps lie outside the box
-// (i = R + 1), only P is kept.  CHECK: some lane of the warp has a source without gradient, whose
-// taps contribute nothing.  A chunk is loaded one source before the first that reaches it and
-// stored after the last.
+// (i = R + 1), only P is kept.  CHECK: some lane of the warp has a source in the image's columns without
+// gradient, whose taps contribute nothing.  (A lane right of the image needs no check: its threshold is NaN, so
+// its terms all go to its column of M, right of the image too, which is not written out.  The last strip of
+// most frames has such lanes; with the check its warp ran another copy of the code than the rest of its CTA, and
+// they waited for each other: 6 frames of 36 x 1576 196 us, 118 without, those of 64 x 1576 114; 34 of
+// 1495 x 1015 at radius 10 3.89 ms and 3.77.)  A chunk is loaded one source before the first that reaches
+// it and stored after the last.
 template <int R, int J, bool CHECK>
 __device__ __forceinline__ void pair_column(float* __restrict__ P, float* __restrict__ M,
                                             const float2* __restrict__ wt, float fi, const float (&gx)[PairLayout<R>::K],
@@ -343,13 +347,13 @@ __global__ void __launch_bounds__(32 * PairLayout<R>::max_warps, 1) fht_rgc_pair
                 gy[y] = ok ? Gy * inv + 0.f : 0.f;  // + 0: -0 becomes +0
                 const bool zero = gx[y] == 0.f && gy[y] == 0.f;
                 some |= !zero;
-                none |= zero;
+                none |= zero && in;  // a lane right of the image: pair_column
                 al = bl, ac = bc, ar = br;
                 bl = cl, bc = cc, br = cr;
             }
             // the next block's rows into L1 while this block's taps run
             for (int y = Y0 + K + 1; y <= Y0 + 2 * K; ++y) asm volatile("prefetch.global.L1 [%0];" ::"l"(row(y) + xc));
-            if (__any_sync(0xffffffffu, none)) {
+            if (__any_sync(0xffffffffu, none || !work)) {  // a warp without work: none of its sources has a gradient
                 if (__any_sync(0xffffffffu, some))
                     pair_block<R, true>(a, sP, sM, swt, lane, gx, gy);
                 else
