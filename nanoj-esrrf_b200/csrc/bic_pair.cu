@@ -145,8 +145,8 @@ __device__ __forceinline__ void load_m(float (&d)[M], const float* s) {
     if constexpr (M == 4) d[2] = v.z, d[3] = v.w;
 }
 
-// The same for the two cells at either end of every row, one pixel a thread (32 rows M 2, 8 rows M 4 a
-// CTA): they are sampled bilinearly at the border, which would hold up the warps of every row.
+// The same for the two cells at either end of every row, one pixel a thread (16 rows at M 2, 8 at M 4
+// a CTA): they are sampled bilinearly at the border, which would hold up the warps of every row.
 template <int M, int SENS>
 __device__ __noinline__ void ends(const BicCumArgs& a) {
     constexpr int kEnds = 4 * M, kRows = 128 / kEnds;
@@ -412,7 +412,9 @@ PairShape shape_of(const BicPairArgs& p, int M, int F, int sms) {
 // rows, 0.13 from 400 on, for 808 instructions a row; the tabulated kernel 6.5 us a CTA and frame with
 // four CTAs an SM at 64 taps, and its gradient kernels.  Measured, one launch with its gradients: 25 of
 // 512 x 512 at M4 2.1 ms against 5.4, 20 frames of 120 x 100 at M4 141 us / 229, 12 of 90 x 80 at M2 (radius
-// 3) 85 / 102, 12 of 37 x 29 at M4 87 / 63, 12 of 60 x 50 at M4 (radius 3) 188 / 128.
+// 3) 85 / 102, 12 of 37 x 29 at M4 87 / 63, 12 of 60 x 50 at M4 (radius 3) 188 / 128.  Of 251 launches that it
+// gives to this form, drawn from 4 x 4 to 700 x 700 pixels, radii 0.5 to 4 and 1 to 32 frames, ten are slower, by
+// 3 to 22 % of 40 to 120 us (eight of them at radius 0.5, 24 taps); the others take 0.64 of the tabulated form's time.
 bool bic_pair_pays(const BicPairTables& t, int w, int h, int M, int F) {
     if (t.I < 1 || F > 65535 || (2L * w + 31) / 32 * F > (1 << 26)) return false;
     int dev = 0;

@@ -9,23 +9,23 @@
 // independent taps take).  So here threads own sources and scatter into their outputs:
 //
 //  * A warp owns a strip of 32 source columns, one lane per column, and walks it downwards in
-//    blocks of 8 rows whose unit gradients it holds in registers.
+//    blocks of K rows (12 up to radius 8, 8 above) whose unit gradients it holds in registers.
 //  * For each column distance i the lane adds its terms to two columns of outputs, at X - i (tile P,
-//    taps (i, j)) and X + i (tile M, the opposite taps), held in registers over all 8 sources x
-//    2J + 1 row distances: 8 + 2J rows each, read from and written back to shared memory once per
+//    taps (i, j)) and X + i (tile M, the opposite taps), held in registers over all K sources x
+//    2J + 1 row distances: K + 2J rows each, read from and written back to shared memory once per
 //    i, four rows at a time.  The lane's two columns move by one with each i, so lanes pass the
 //    columns on through shared memory; tiles P and M are separate, so that both are loaded before
 //    the taps and no lane waits for another's half.  The columns of a tile are an odd number of
 //    16-byte chunks apart: a warp's 128-bit accesses are free of bank conflicts.
-//  * The rows of the tiles form a ring of 4-row chunks: after each block the two oldest chunks are
-//    complete for this strip's sources; they are written out and cleared.
+//  * After each block the tiles' first K rows are complete for this strip's sources: they are written out
+//    and the other rows move up, in 4-row chunks.
 //  * Outputs within R + 1 columns of a strip's edge also receive terms from the neighbouring strip's
 //    sources.  Each strip writes its own 32 columns to the plane `own` and the rest to the plane
 //    `edge` (every element of it has one writer); the reader adds the two.
 // Taps without a partner in the box [-R, R + 1] (column or row R + 1) go through the same code with
 // one of the two additions left out.
 //
-// Bound: instruction issue.  512 x 512 frames at M4, radius 1.5 (254 taps), 34 a launch: 1.174e8 warp
+// Bound: instruction issue.  512 x 512 frames at M4, radius 1.5 (254 taps), 34 a launch: 1.176e8 warp
 // instructions per frame (the fused tile kernel, fht_fused.cuh: 2.214e8), 0.78 issued per cycle and
 // scheduler, 5.02 ms against 8.25; the cumulants (rgc_pair.cu) take 0.35 ms more.  What the split is
 // made of, each measured on that launch:

@@ -69,6 +69,7 @@ struct CumArgs {
 // around it at its end; the intensity is summed once for all sensitivities.  100 frames of 1024 x 1024,
 // three sensitivities, three blocks of which two hold each frame: 1.33 ms with sums for every block and
 // two sensitivities a launch, 0.79 ms with stretches and three, 0.46 ms with the powers formed once.
+// Four CTAs an SM leave 128 registers: three sensitivities spill 128 bytes (any others than 1 to 4: 176), two 48 (16).
 // SMALL: every sensitivity is 1, 2, 3 or 4, whose powers (dev::cglh_power's) are formed once a frame.
 template <int NS, bool SMALL>
 __global__ void __launch_bounds__(128, 4) sweep_cumulants_kernel(CumArgs a) {
